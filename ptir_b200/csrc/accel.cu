@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(kCollapseThreads) k_collapse4(int n, const flo
 __global__ void k_emit4(int n, const float4* __restrict__ nodes, const float4* __restrict__ sbox,
                         const unsigned* __restrict__ order, const int* __restrict__ wsrc,
                         const int* __restrict__ wchild, const unsigned* __restrict__ wcount,
-                        float4* __restrict__ nodes4) {
+                        float4* __restrict__ nodes4, float4* __restrict__ quads) {
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= n - 1 || (unsigned)w >= *wcount) return;
     float lx[4], ly[4], lz[4], hx[4], hy[4], hz[4], km[4];
@@ -577,6 +577,11 @@ __global__ void k_emit4(int n, const float4* __restrict__ nodes, const float4* _
     out[5] = make_float4(hz[0], hz[1], hz[2], hz[3]);
     out[6] = make_float4(__int_as_float(ch[0]), __int_as_float(ch[1]), __int_as_float(ch[2]), __int_as_float(ch[3]));
     out[7] = make_float4(km[0], km[1], km[2], km[3]);
+    float4* quad = quads + 8 * (size_t)w;
+    for (int k = 0; k < 4; ++k) {
+        quad[2 * k] = make_float4(lx[k], ly[k], lz[k], hx[k]);
+        quad[2 * k + 1] = make_float4(hy[k], hz[k], __int_as_float(ch[k]), km[k]);
+    }
 }
 
 template <class T>
@@ -716,6 +721,7 @@ cudaError_t accel_build(AccelState& st, const AccelBuildOptions& opt, const floa
         PTIR_TRY(grow(st.wchild, 4 * cap, s));
         if (!st.wcount) PTIR_TRY(cudaMallocAsync(reinterpret_cast<void**>(&st.wcount), sizeof(unsigned), s));
         PTIR_TRY(grow(st.nodes4, 8 * (cap > 1 ? cap - 1 : 1), s));
+        PTIR_TRY(grow(st.quads, 8 * (cap > 1 ? cap - 1 : 1), s));
         st.capacity = cap;
         st.valid = false;
     }
@@ -764,7 +770,7 @@ cudaError_t accel_build(AccelState& st, const AccelBuildOptions& opt, const floa
             PTIR_TRY(cudaGetLastError());
         }
         k_emit4<<<(unsigned)((n - 1 + T - 1) / T), T, 0, s>>>(n, st.nodes, st.box, st.ids[1], st.wsrc, st.wchild,
-                                                             st.wcount, st.nodes4);
+                                                             st.wcount, st.nodes4, st.quads);
         PTIR_TRY(cudaGetLastError());
     }
     st.valid = true;
@@ -794,6 +800,7 @@ void accel_free(AccelState& st) {
     rel(st.wchild);
     rel(st.wcount);
     rel(st.nodes4);
+    rel(st.quads);
     if (st.ploc_host) cudaFreeHost(st.ploc_host);
     st = AccelState();
 }

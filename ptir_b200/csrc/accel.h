@@ -39,13 +39,14 @@ struct AccelState {
     int* wsrc = nullptr;        // [(n-1)*4] children of each 4-wide node as binary references (refits)
     int* wchild = nullptr;      // [(n-1)*4] the same children as 4-wide node indices or leaves
     unsigned* wcount = nullptr; // number of 4-wide nodes
-    float4* nodes4 = nullptr;   // [(n-1)*8] 4-wide nodes traversed by the tracer
+    float4* nodes4 = nullptr;   // [(n-1)*8] 4-wide nodes traversed by the tracer, one lane a ray
+    float4* quads = nullptr;    // [(n-1)*8] the same nodes child by child, four lanes a ray
     void* sort_temp = nullptr;
     size_t sort_temp_bytes = 0;
     unsigned* ploc_host = nullptr;  // pinned [2]: cluster count and next node index read back by a PLOC build
     size_t capacity = 0;        // Gaussians the buffers can hold
 
-    AccelView view() const { return AccelView{nodes4, leaves, bounds, valid ? n : 0, 0.0f}; }
+    AccelView view() const { return AccelView{nodes4, quads, leaves, bounds, valid ? n : 0, 0.0f}; }
 };
 
 // Build (rebuild != 0 or topology unusable) or refit the structure from per-Gaussian

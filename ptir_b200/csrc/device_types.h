@@ -21,6 +21,7 @@ constexpr int kNoChild = (int)0x80000000;
 
 struct AccelView {
     const float4* nodes;  // 4-wide nodes
+    const float4* quads;  // the same nodes child by child: 4 x (lo.xyz hi.x | hi.yz child kmax)
     const float4* leaves;
     const float4* bounds;  // [2]: scene AABB lo.xyz, hi.xyz (union of the instance AABBs)
     int n;                 // number of Gaussians (leaves)

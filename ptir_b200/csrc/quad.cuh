@@ -1,0 +1,209 @@
+// Traversal with four lanes a ray ("quad"): the calls of traverse.cuh, decision for decision, with the
+// work of one node visit spread over the lanes instead of looped over.
+//
+// Lane c of a quad tests child c of the 4-wide node and, when that is a leaf, the leaf's candidate
+// test, so the leaf tests of a visit run side by side; the k-buffer is spread over the quad (lane c
+// holds entries c K/4 to (c+1) K/4 - 1); the order of the children comes from comparing keys across
+// the quad, and up to four stack entries are popped at a time. A visit decides what the one-lane visit
+// decides: the leaf tests of a node see the K-th distance as it was before the node, but an entry at or
+// past the current K-th distance enters the sorted buffer nowhere, which is the one-lane test's
+// rejection; children are visited and stacked in the same order.
+//
+// Bound: latency. A visit is a chain of a node load, box tests, leaf loads and tests, insertions and
+// the descent. With one lane a ray that chain took 0.9 to 1.2 us a visit (leaf tests one after the
+// other, an insertion a chain of 16 selects, 32 registers of k-buffer), and the longest of a launch's
+// rays (up to 5000 visits on a million Gaussians) set the time of every bounce stage. See k_wf_trace_quad.
+#pragma once
+
+#include "leaf.cuh"
+
+namespace ptir {
+
+constexpr int kQuadStackPad = 2;  // entries: quads of a warp start in different shared-memory banks
+
+// A trace call of a quad's ray. Everything but the k-buffer part (kt, kid) is the same in its four lanes.
+template <int K>
+struct QuadTrace {
+    static constexpr int L = K / 4;  // k-buffer entries a lane
+    float3 inv;
+    float tmin, tend;
+    float slack, cap, floor;  // as TraceState
+    float tk;                 // the K-th distance
+    int node, sp;
+    float kt[L];
+    unsigned kid[L];
+};
+
+// Insert (ts, id) into the quad's sorted k-buffer, behind equal distances; kFarT goes nowhere. Called by
+// every lane of `mask` with its quad's entry. kbuf_insert's chain of swaps moves the first entry of a run of
+// equal distances behind the run when something is inserted before it (an entry passes only what is
+// strictly farther); so does this, for runs that lie in at most two lanes: an entry moves on only past a
+// strictly nearer one (`moves`), and what arrives behind a run is the run's first (`run`).
+template <int K>
+PTIR_DEV void quad_insert(QuadTrace<K>& t, float ts, unsigned id, unsigned c, unsigned mask) {
+    constexpr int L = QuadTrace<K>::L;
+    unsigned run[L];
+#pragma unroll
+    for (int j = 0; j < L; ++j) run[j] = (j > 0 && t.kt[j] == t.kt[j > 0 ? j - 1 : 0]) ? run[j > 0 ? j - 1 : 0] : t.kid[j];
+    float pt = __shfl_up_sync(mask, t.kt[L - 1], 1, 4);
+    const unsigned pid = __shfl_up_sync(mask, run[L - 1], 1, 4);
+    if (c == 0) pt = -kFarT;  // nothing moves in from before the first lane
+#pragma unroll
+    for (int j = L - 1; j >= 0; --j) {
+        const float prev = j > 0 ? t.kt[j > 0 ? j - 1 : 0] : pt;
+        unsigned prev_id = j > 0 ? run[j > 0 ? j - 1 : 0] : pid;
+        // the run of entry j - 1 reaches back over the whole part: it may start in the lane before
+        if (j > 0 && t.kt[j > 0 ? j - 1 : 0] == t.kt[0] && t.kt[0] == pt) prev_id = pid;
+        const float in = fmaxf(prev, ts);
+        const bool moves = in < t.kt[j];
+        t.kid[j] = moves ? (ts < prev ? prev_id : id) : t.kid[j];
+        t.kt[j] = moves ? in : t.kt[j];
+    }
+}
+
+// number of filled entries of this lane's part
+template <int K>
+PTIR_DEV unsigned quad_count(const QuadTrace<K>& t) {
+    return kbuf_count(t.kt);
+}
+
+// trace_start for a quad: true when node visits remain
+template <int K>
+PTIR_DEV bool quad_start(const AccelView& A, float3 o, float3 d, float tmin, float tend, QuadTrace<K>& t,
+                         TraceCounters& ctr, unsigned c, float cap) {
+    t.cap = cap;
+    t.floor = -kFarT;
+    t.tk = kFarT;
+    kbuf_clear(t.kt, t.kid);
+    if (c == 0) ++ctr.calls;
+    if (A.n <= 0) return false;
+    t.tmin = tmin;
+    t.tend = tend;
+    if (A.n == 1) {
+        if (c == 0) {
+            ++ctr.leaves;
+            float ts;
+            unsigned id;
+            if (leaf_candidate_wide(A, 0, o, d, tmin, tend, kFarT, ts, id, -kFarT)) {
+                t.kt[0] = ts;
+                t.kid[0] = id;
+                ++ctr.candidates;
+            }
+        }
+        return false;
+    }
+    t.inv = make_float3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+    t.slack = A.cull_slack > 0.0f ? A.cull_slack / sqrtf(dot(d, d)) : 0.0f;
+    t.node = 0;
+    t.sp = 0;
+    return true;
+}
+
+// trace_continue for a quad
+template <int K>
+PTIR_DEV void quad_continue(QuadTrace<K>& t, TraceCounters& ctr) {
+    ctr.candidates -= quad_count(t);
+    t.floor = t.cap;
+    t.cap = kFarT;
+    t.node = 0;
+    t.sp = 0;
+}
+
+// One node visit of the quads in `mask` (whole quads, all of them tracing). Returns false when the
+// quad's call is complete. `stack` is the quad's, in shared memory.
+template <int K, bool kSlack>
+PTIR_DEV bool quad_step(const AccelView& A, float3 o, float3 d, QuadTrace<K>& t, StackEntry* stack, unsigned* err,
+                        TraceCounters& ctr, unsigned ln, unsigned mask) {
+    constexpr int L = QuadTrace<K>::L;
+    const unsigned c = ln & 3u, base = ln & 28u;
+    const float3 inv = t.inv;
+    float4 p, q;  // lo.xyz hi.x | hi.yz child kmax
+    ld256(A.quads + 8 * (size_t)t.node + 2 * c, p, q);
+    const int child = __float_as_int(q.z);
+    const bool px = inv.x >= 0.0f, py = inv.y >= 0.0f, pz = inv.z >= 0.0f;
+    // the clipped slab interval of visit_node
+    const float3 oi = make_float3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+    const float a = max3f(fmaf(px ? p.x : p.w, inv.x, -oi.x), fmaf(py ? p.y : q.x, inv.y, -oi.y),
+                          fmaxf(fmaf(pz ? p.z : q.y, inv.z, -oi.z), t.tmin));
+    const float b = min3f(fmaf(px ? p.w : p.x, inv.x, -oi.x), fmaf(py ? q.x : p.y, inv.y, -oi.y),
+                          fminf(fmaf(pz ? q.y : p.z, inv.z, -oi.z), t.tend));
+    const float sl = (kSlack && t.slack > 0.0f) ? q.w * t.slack : 0.0f;
+    const float t0 = kSlack ? a - sl : a;
+    const float key = 15.0f * a + b;
+    float cut = fminf(t.tk, t.cap);
+    const bool hit = child != kNoChild && a <= b && (kSlack ? b + sl : b) >= t.floor && t0 <= cut;
+    if (c == 0) ++ctr.nodes;
+    float ts = kFarT;
+    unsigned id = kNoHit;
+    bool cand = false;
+    if (hit && child < 0) {
+        ++ctr.leaves;
+        cand = leaf_candidate_wide(A, ~child, o, d, t.tmin, t.tend, cut, ts, id, t.floor);
+    }
+    const unsigned cands = __ballot_sync(mask, cand);
+    if (cands) {  // uniform over the mask
+        unsigned mine = (cands >> base) & 15u;
+        do {
+            const unsigned src = base + (mine ? __ffs(mine) - 1 : 0u);
+            const float tin = __shfl_sync(mask, ts, src);
+            const unsigned iin = __shfl_sync(mask, id, src);
+            quad_insert(t, mine ? tin : kFarT, iin, c, mask);
+            mine &= mine - 1u;
+        } while (__any_sync(mask, mine != 0u));
+        t.tk = __shfl_sync(mask, t.kt[L - 1], base + 3u);
+        cut = fminf(t.tk, t.cap);
+    }
+    // descent: the internal children still in front of the cut, nearest key first; the others are stacked
+    // largest key first. Keys are compared as integers (they are not negative) with the child in the two
+    // lowest bits, so that they differ and name their lane.
+    const bool inner = hit && child >= 0 && t0 <= cut;
+    const int ik = inner ? (int)((__float_as_uint(key) & ~3u) | c) : 0x7FFFFFFF;
+    const int k1 = __shfl_xor_sync(mask, ik, 1), k2 = __shfl_xor_sync(mask, ik, 2), k3 = __shfl_xor_sync(mask, ik, 3);
+    const int rank = (k1 < ik ? 1 : 0) + (k2 < ik ? 1 : 0) + (k3 < ik ? 1 : 0);
+    const int best = min(min(ik, k1), min(k2, k3));
+    const int np = __popc((__ballot_sync(mask, inner) >> base) & 15u) - 1;  // stacked children
+    const int next = __shfl_sync(mask, child, base + (best & 3));
+    bool more = true, pop = np < 0;
+    if (!pop) {
+        if (t.sp + np > kStackDepth) {
+            if (c == 0) atomicOr(err, kErrStackOverflow);
+            more = false;
+        } else {
+            if (inner && rank > 0) stack[t.sp + np - rank] = make_int2(child, __float_as_int(t0));
+            t.sp += np;
+            t.node = next;
+        }
+    }
+    __syncwarp(mask);
+    // pop the next subtree that can still hold a nearer candidate, four entries at a time
+    while (__any_sync(mask, pop)) {
+        const int i = t.sp - 1 - (int)c;
+        StackEntry e = make_int2(0, 0);
+        bool ok = false;
+        if (pop && i >= 0) {
+            e = stack[i];
+            ok = __int_as_float(e.y) <= cut;
+        }
+        const unsigned om = (__ballot_sync(mask, ok) >> base) & 15u;
+        const unsigned first = om ? __ffs(om) - 1 : 0u;
+        const int popped = __shfl_sync(mask, e.x, base + first);
+        if (pop) {
+            if (om) {
+                t.node = popped;
+                t.sp -= 1 + (int)first;
+                pop = false;
+            } else {
+                t.sp -= 4;
+                if (t.sp <= 0) {
+                    pop = false;
+                    more = false;
+                }
+            }
+        }
+    }
+    // (the entries just read are overwritten only after the next visit's ballots)
+    if (!more) ctr.candidates += quad_count(t);
+    return more;
+}
+
+}  // namespace ptir

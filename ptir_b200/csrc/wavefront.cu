@@ -23,6 +23,7 @@
 
 #include "radix_sort.cuh"
 #include "path.cuh"
+#include "quad_path.cuh"
 #include "wavefront.h"
 
 namespace ptir {
@@ -227,6 +228,12 @@ constexpr int trace_regs(int K) { return K > 16 ? 128 : 96; }
 // of them continued), against 145.5 ms at 1.5 and 143.2 ms at 3.
 constexpr float kSeedSpan = 2.0f;
 
+// Rays up to which an intersection launch takes four lanes a ray. Measured against one lane (intersection stage,
+// ms): 1.93 -> 0.93 at 16k rays over 10k Gaussians, 36.2 -> 23.3 at 90k over 300k, 9.3 -> 7.7 at 278k
+// primary and 80k bounce rays over 30k; all of a launch of 786k primary and about 200k bounce rays over 1M
+// took 157.6 against 147.8, and with the line at 262,144 instead of 131,072 150.4.
+constexpr unsigned kQuadRays = 1u << 17;
+
 //
 // With K = 32 a traversal stands for two of the reference's 16-candidate rounds (the rounds of
 // pathTracer.cuh:216-311): its first 16 candidates are the first round, and its last 16 are the
@@ -241,7 +248,8 @@ constexpr float kSeedSpan = 2.0f;
 // applies the exact-candidate cull slack (only tracers with exact_candidates launch it).
 template <int K, bool kMark, bool kSelfOcc, bool kResume, bool kSlack>
 __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis, WfView W, int in_q,
-                                                      const unsigned* items, int out_q, unsigned cursor, int refill) {
+                                                      const unsigned* items, int out_q, unsigned cursor, int refill,
+                                                      unsigned quad_rays) {
     constexpr bool kPair = K == 32;  // traversals gather two 16-candidate rounds (leaf-index k-buffer)
     static_assert(!(kPair && kResume), "resumed calls take the 16-candidate rounds one by one");
     static_assert(!(kSlack && kResume), "the exact-candidate slack is applied by the rounds from the root");
@@ -259,6 +267,7 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
     constexpr unsigned kFull = 0xFFFFFFFFu;
     enum : int { kIdle = 0, kTracing = 1, kReady = 2 };
     const unsigned count = W.count[in_q];
+    if (count <= quad_rays) return;  // the quads' launch
     int phase = kIdle;
     unsigned q = 0;
     int rounds = 0;
@@ -411,6 +420,153 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
                 pk.save(c);
             }
         }
+        if (out_q >= 0) push(W.q[out_q], W.count + out_q, q, done);
+    }
+    flush_counters(P, ctr);
+}
+
+// ---------------------------------------------------------------------------------------
+// intersection, four lanes a ray
+
+// Shared memory of a quad: its traversal stack (the staging of quad_composite lies over it: no traversal
+// is in progress then) and its compositing state.
+struct QuadSlot {
+    StackEntry stack[kStackDepth + kQuadStackPad];
+    QuadComposite comp;
+};
+static_assert(sizeof(float4) * kQuadStage <= sizeof(StackEntry) * kStackDepth, "the staging fits the stack");
+static_assert(sizeof(QuadSlot) % 16 == 0, "float4 members");
+
+constexpr size_t quad_smem(int block) { return sizeof(QuadSlot) * (size_t)(block / 4); }
+
+// Rays a warp carries: all eight quads, or fewer when the queue holds less than the grid's quads, so that
+// a small launch spreads over all warps and no ray waits for another's.
+PTIR_DEV unsigned quads_in_use(unsigned count) {
+    const unsigned warps = gridDim.x * (blockDim.x >> 5);
+    return min(8u, max(1u, (count + warps - 1u) / warps));
+}
+
+// k_wf_trace for the rounds from the root (K <= 16) of small launches, a quad of lanes per segment (quad.cuh).
+// The decisions, their order and the compositing are k_wf_trace's, and no first round is seeded: a quad rarely
+// sees more than a few segments. A small launch is bound by the chain of its slowest ray, which one lane walks
+// at about 1 us a visit; here the visit's parts run side by side (preview of 2,867 rays over 2k Gaussians:
+// 1.42 -> 0.49 ms in the stage). 96 registers hold the visit without spills: 23.6 ms at 90k rays over 300k
+// Gaussians, against 26.1 at 72 and 25.9 at 64, where spills cost more than the warps gain.
+template <int K, bool kMark, bool kSelfOcc, bool kSlack>
+__global__ void __maxnreg__(96) k_wf_trace_quad(TraceParams P, float* vis, WfView W, int in_q, const unsigned* items,
+                                                int out_q, unsigned cursor, int refill, unsigned quad_rays) {
+    extern __shared__ float4 quad_mem[];
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    enum : int { kIdle = 0, kTracing = 1, kReady = 2 };
+    const unsigned ln = lane(), c = ln & 3u, base = ln & 28u;
+    QuadSlot& slot = reinterpret_cast<QuadSlot*>(quad_mem)[threadIdx.x >> 2];
+    TraceCounters ctr = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const unsigned count = W.count[in_q];
+    if (count > quad_rays) return;
+    const bool in_use = (ln >> 2) < quads_in_use(count);
+    int phase = kIdle;
+    unsigned q = 0;
+    int rounds = 0;
+    bool drained = false, seeded = false;
+    float3 ro = f3(0.0f), rd = f3(0.0f);
+    QuadTrace<K> t;
+    t.tk = kFarT;
+    // next trace call of the quad's segment, or ready with nothing found when it is complete
+    auto next_call = [&](float span) {
+        t.tk = kFarT;
+        const QuadComposite& s = slot.comp;
+        bool call = quad_open(P, s);
+        if (call && ++rounds > kMaxRounds + 1) {
+            if (c == 0) atomicOr(P.error_word, kErrLoopBound);
+            call = false;
+        }
+        phase = kReady;
+        if (!call) {
+            kbuf_clear(t.kt, t.kid);
+            return;
+        }
+        const float tmin = s.last_hit + 1e-9f, tend = s.clip_end + 1e-9f;
+        float cap = kFarT;
+        seeded = false;
+        if (K == 16 && span > 0.0f) {
+            cap = tmin + kSeedSpan * span;
+            seeded = cap < tend;
+            if (!seeded) cap = kFarT;
+        }
+        if (quad_start(P.accel, ro, rd, tmin, tend, t, ctr, c, cap)) phase = kTracing;
+    };
+    while (true) {
+        // refill the idle quads
+        const unsigned idle = __ballot_sync(kFull, phase == kIdle && in_use && c == 0);
+        if (!drained && idle) {
+            const unsigned n_idle = __popc(idle);
+            unsigned first = 0;
+            if (ln == 0) first = atomicAdd(W.cursor + cursor, n_idle);
+            first = __shfl_sync(kFull, first, 0);
+            drained = first + n_idle >= count;
+            const unsigned i = first + __popc(idle & ((1u << base) - 1u));
+            const bool take = phase == kIdle && in_use && i < count;
+            const unsigned taking = __ballot_sync(kFull, take);
+            if (take) {
+                q = items[i];
+                ro = W.seg[q].o;
+                rd = W.seg[q].d;
+                rounds = 0;
+                quad_composite_begin(P, slot.comp, ro, rd, c, taking);
+                if (c == 0) ++ctr.segments;
+                next_call(0.0f);
+            }
+        }
+        const unsigned busy = __ballot_sync(kFull, phase != kIdle && c == 0);
+        if (!busy) {
+            if (drained) break;
+            continue;
+        }
+        // traverse until enough quads wait
+        while (true) {
+            const unsigned tracing = __ballot_sync(kFull, phase == kTracing);
+            if (!tracing || __popc(busy) - (__popc(tracing) >> 2) >= (drained ? 1 : refill)) break;
+            if (phase == kTracing && !quad_step<K, kSlack>(P.accel, ro, rd, t, slot.stack, P.error_word, ctr, ln, tracing)) {
+                if (seeded && t.tk >= kFarT) {
+                    seeded = false;
+                    quad_continue(t, ctr);
+                } else {
+                    phase = kReady;
+                }
+            }
+        }
+        // composite the finished calls; hand on the finished segments
+        bool done = false;
+        const unsigned ready = __ballot_sync(kFull, phase == kReady);
+        if (phase == kReady) {
+            const float t_first = __shfl_sync(ready, t.kt[0], base);
+            const float t_last = __shfl_sync(ready, t.kt[QuadTrace<K>::L - 1], base + 3u);
+            bool complete = true;
+            const unsigned found = __ballot_sync(ready, t_first < kFarT);
+            if (t_first < kFarT) {
+                quad_composite<kSelfOcc>(P, ctr, slot.comp, reinterpret_cast<float4*>(slot.stack), t, ro, rd,
+                                         kMark ? vis : nullptr, ln, found);
+                // a k-buffer that is not full held every candidate of the call: a later call finds none
+                if (t_last < kFarT) {
+                    next_call(t_last - t_first);
+                    complete = phase == kReady;
+                }
+            }
+            if (complete) {
+                if (c == 0) {
+                    Composite cm;
+                    quad_composite_gather(slot.comp, cm, ro, rd);
+                    Segment s;
+                    Pcg32 rng = load_rng(W, q);
+                    composite_end(P, cm, W.seg[q].scatter_pdf, W.seg[q].light_pdf, s, rng);
+                    W.seg[q] = s;
+                    store_rng(W, q, rng);
+                    done = true;
+                }
+                phase = kIdle;
+            }
+        }
+        __syncwarp();
         if (out_q >= 0) push(W.q[out_q], W.count + out_q, q, done);
     }
     flush_counters(P, ctr);
@@ -948,34 +1104,61 @@ static bool use_resume(const WavefrontTuning& tune) {
     return K <= 16 && tune.resume_isect && !tune.exact_candidates;
 }
 
-// the intersection kernel of a launch: resumed rounds, the exact-candidate slack, or neither
-template <int K, bool kMark, bool kSelfOcc>
-static const void* trace_kernel(bool resume, bool slack) {
-    if constexpr (K <= 16) {
-        if (resume) return (const void*)k_wf_trace<K, kMark, kSelfOcc, true, false>;
-    }
-    if (slack) return (const void*)k_wf_trace<K, kMark, kSelfOcc, false, true>;
-    return (const void*)k_wf_trace<K, kMark, kSelfOcc, false, false>;
-}
+// An intersection launch: the kernels of its k-buffer size and options, and their persistent grids. Rounds from
+// the root with K <= 16 take four lanes a ray (k_wf_trace_quad) in a launch of up to kQuadRays rays and one lane
+// a ray (k_wf_trace) in a larger one; resumed rounds and K = 32 always take one.
+struct TraceLaunch {
+    const void* lane_fn = nullptr;
+    const void* quad_fn = nullptr;
+    int block, lane_refill, quad_refill, lane_grid = 0, quad_grid = 0;
+};
 
 template <int K, bool kMark, bool kSelfOcc>
-static int trace_grid(bool resume, bool slack, int B) {
-    return grid_cached(trace_kernel<K, kMark, kSelfOcc>(resume, slack), B);
-}
-
-template <int K, bool kMark, bool kSelfOcc>
-static void launch_trace(bool resume, bool slack, int grid, int B, cudaStream_t s, const TraceParams& q, float* vis,
-                         const WfView& W, int in_q, const unsigned* items, int out_q, unsigned cursor, int R) {
+static TraceLaunch trace_launch(const WavefrontTuning& tune, bool resume) {
+    TraceLaunch l;
+    l.block = tune.block;
+    l.lane_refill = tune.refill_lanes;
+    l.quad_refill = (tune.refill_lanes + 3) / 4;
+    const bool slack = tune.exact_candidates;
     if constexpr (K <= 16) {
         if (resume) {
-            k_wf_trace<K, kMark, kSelfOcc, true, false><<<grid, B, 0, s>>>(q, vis, W, in_q, items, out_q, cursor, R);
-            return;
+            l.lane_fn = (const void*)k_wf_trace<K, kMark, kSelfOcc, true, false>;
+        } else {
+            l.lane_fn = slack ? (const void*)k_wf_trace<K, kMark, kSelfOcc, false, true>
+                              : (const void*)k_wf_trace<K, kMark, kSelfOcc, false, false>;
+            l.quad_fn = slack ? (const void*)k_wf_trace_quad<K, kMark, kSelfOcc, true>
+                              : (const void*)k_wf_trace_quad<K, kMark, kSelfOcc, false>;
         }
+    } else {
+        l.lane_fn = slack ? (const void*)k_wf_trace<K, kMark, kSelfOcc, false, true>
+                          : (const void*)k_wf_trace<K, kMark, kSelfOcc, false, false>;
     }
-    if (slack)
-        k_wf_trace<K, kMark, kSelfOcc, false, true><<<grid, B, 0, s>>>(q, vis, W, in_q, items, out_q, cursor, R);
-    else
-        k_wf_trace<K, kMark, kSelfOcc, false, false><<<grid, B, 0, s>>>(q, vis, W, in_q, items, out_q, cursor, R);
+    l.lane_grid = grid_cached(l.lane_fn, l.block);
+    if (l.quad_fn) l.quad_grid = grid_cached(l.quad_fn, l.block, quad_smem(l.block));
+    return l;
+}
+
+// The intersection of queue in_q, which holds at most `rays` rays. How many it does hold only the device knows,
+// so a queue that might be on either side of kQuadRays gets both launches, and the kernel that it is not for
+// returns at once.
+static void run_trace(const TraceLaunch& l, long long rays, const TraceParams& q, float* vis, const WfView& W, int in_q,
+                      const unsigned* items, int out_q, unsigned cursor, cudaStream_t s) {
+    TraceParams p = q;
+    WfView w = W;
+    const auto blocks = [&](int grid, long long per_block) {
+        return dim3((unsigned)std::max<long long>(1, std::min<long long>(grid, (rays + per_block - 1) / per_block)));
+    };
+    unsigned quad_rays = l.quad_fn ? kQuadRays : 0u;
+    int refill;
+    void* args[] = {&p, &vis, &w, &in_q, &items, &out_q, &cursor, &refill, &quad_rays};
+    if (l.quad_fn) {
+        refill = l.quad_refill;
+        cudaLaunchKernel(l.quad_fn, blocks(l.quad_grid, l.block / 32), dim3((unsigned)l.block), args, quad_smem(l.block), s);
+    }
+    if (rays > (long long)quad_rays) {
+        refill = l.lane_refill;
+        cudaLaunchKernel(l.lane_fn, blocks(l.lane_grid, l.block), dim3((unsigned)l.block), args, 0, s);
+    }
 }
 
 template <int K>
@@ -990,10 +1173,9 @@ static cudaError_t run_fwd(const TraceParams& p, const FwdOutputs& o, WavefrontB
     const int g_camera = grid_cached((const void*)k_wf_camera, B);
     const int g_primary = grid_cached((const void*)k_wf_fwd_primary<K>, B);
     const int g_bounce = grid_cached((const void*)k_wf_fwd_bounce<K>, B);
-    const bool resume = use_resume<K>(tune), slack = tune.exact_candidates;
-    const int g_trace0 = trace_grid<K, true, false>(resume, slack, B);
-    const int g_trace = trace_grid<K, true, true>(resume, slack, B);
-    if (resume && (e = frontier_reserve(b, std::max(g_trace0, g_trace) * B, s)) != cudaSuccess) return e;
+    const bool resume = use_resume<K>(tune);
+    const TraceLaunch trace0 = trace_launch<K, true, false>(tune, resume), trace = trace_launch<K, true, true>(tune, resume);
+    if (resume && (e = frontier_reserve(b, (size_t)std::max(trace0.lane_grid, trace.lane_grid) * B, s)) != cudaSuccess) return e;
     const unsigned mb = p.render_opts ? std::min(p.max_bounces, 2u) : p.max_bounces;
     if (kFirstBounceCursor + 2u * mb > (unsigned)kNumCursors) return cudaErrorInvalidValue;
     for (unsigned long long t0 = 0; t0 < tiles; t0 += chunk_tiles) {
@@ -1006,8 +1188,7 @@ static cudaError_t run_fwd(const TraceParams& p, const FwdOutputs& o, WavefrontB
             k_wf_camera<<<std::min(g_camera, cap), B, 0, s>>>(q, W);
         });
         sc.run(kStageIntersect, p, s, [&](const TraceParams& q) {
-            launch_trace<K, true, false>(resume, slack, std::min(g_trace0, cap), B, s, q, o.visibility, W, kQIsect,
-                                         W.q[kQIsect], -1, 1, R);
+            run_trace(trace0, (long long)nt * 32, q, o.visibility, W, kQIsect, W.q[kQIsect], -1, 1, s);
         });
         sc.run(kStageShading, p, s, [&](const TraceParams& q) {
             k_wf_fwd_primary<K><<<std::min(g_primary, cap), B, 0, s>>>(q, o, W);
@@ -1028,8 +1209,7 @@ static cudaError_t run_fwd(const TraceParams& p, const FwdOutputs& o, WavefrontB
             cudaMemsetAsync(W.count + kQBounce, 0, sizeof(unsigned), s);
             const unsigned* items = sort_queue(p, b, W, tune, sc, s);
             sc.run(kStageIntersect, p, s, [&](const TraceParams& q) {
-                launch_trace<K, true, true>(resume, slack, g_trace, B, s, q, o.visibility, W, kQIsect, items, kQBounce,
-                                            cursor, R);
+                run_trace(trace, (long long)nt * 32, q, o.visibility, W, kQIsect, items, kQBounce, cursor, s);
             });
             ++cursor;
         }
@@ -1051,12 +1231,11 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
     const int g_camera = grid_cached((const void*)k_wf_camera, B);
     const int g_primary = grid_cached((const void*)k_wb_primary<K>, B);
     const int g_bounce = grid_cached((const void*)k_wb_bounce<K>, B);
-    const bool resume = use_resume<K>(tune), slack = tune.exact_candidates;
+    const bool resume = use_resume<K>(tune);
     const bool resume_replay = K <= 16 && tune.resume_replay;
-    const int g_trace0 = trace_grid<K, false, false>(resume, slack, B);
-    const int g_trace = trace_grid<K, false, true>(resume, slack, B);
+    const TraceLaunch trace0 = trace_launch<K, false, false>(tune, resume), trace = trace_launch<K, false, true>(tune, resume);
     const int g_replay = grid_cached((const void*)k_wb_replay<K>, B);
-    const int g_front = std::max(resume ? std::max(g_trace0, g_trace) : 0, resume_replay ? g_replay : 0);
+    const int g_front = std::max(resume ? std::max(trace0.lane_grid, trace.lane_grid) : 0, resume_replay ? g_replay : 0);
     if (g_front > 0 && (e = frontier_reserve(b, (size_t)g_front * B, s)) != cudaSuccess) return e;
     const unsigned mb = p.render_opts ? std::min(p.max_bounces, 2u) : p.max_bounces;
     if (kFirstBounceCursor + 3u * mb > (unsigned)kNumCursors) return cudaErrorInvalidValue;
@@ -1070,8 +1249,7 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
             k_wf_camera<<<std::min(g_camera, cap), B, 0, s>>>(q, W);
         });
         sc.run(kStageIntersect, p, s, [&](const TraceParams& q) {
-            launch_trace<K, false, false>(resume, slack, std::min(g_trace0, cap), B, s, q, nullptr, W, kQIsect,
-                                          W.q[kQIsect], -1, 1, R);
+            run_trace(trace0, (long long)nt * 32, q, nullptr, W, kQIsect, W.q[kQIsect], -1, 1, s);
         });
         sc.run(kStageShading, p, s, [&](const TraceParams& q) {
             k_wb_primary<K><<<std::min(g_primary, cap), B, 0, s>>>(q, bi, W);
@@ -1097,8 +1275,7 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
             cudaMemsetAsync(W.count + kQBounce, 0, sizeof(unsigned), s);
             const unsigned* items = sort_queue(p, b, W, tune, sc, s);
             sc.run(kStageIntersect, p, s, [&](const TraceParams& q) {
-                launch_trace<K, false, true>(resume, slack, g_trace, B, s, q, nullptr, W, kQIsect, items, kQBounce,
-                                             cursor, R);
+                run_trace(trace, (long long)nt * 32, q, nullptr, W, kQIsect, items, kQBounce, cursor, s);
             });
             ++cursor;
         }
