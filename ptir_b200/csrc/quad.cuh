@@ -19,7 +19,7 @@
 
 namespace ptir {
 
-constexpr int kQuadStackPad = 2;  // entries: quads of a warp start in different shared-memory banks
+constexpr int kQuadStackEntries = kStackDepth + 2;  // quads of a warp start in different shared-memory banks
 
 // A trace call of a quad's ray. Everything but the k-buffer part (kt, kid) is the same in its four lanes.
 template <int K>

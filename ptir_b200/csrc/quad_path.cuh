@@ -167,4 +167,42 @@ PTIR_DEV void quad_composite_gather(const QuadComposite& s, Composite& c, float3
     c.hit = s.hit != 0.0f;
 }
 
+// The shadow walk over the batch of the finished call of each quad in `mask` (shadow_occluded in path.cuh), in
+// the batch's order with the ray's own draws, which all four lanes make: whether a hit occludes the ray; else
+// `batch_end` is raised to the farthest hit walked.
+template <int K>
+PTIR_DEV bool quad_shadow_walk(const TraceParams& P, const QuadTrace<K>& t, float3 o, float3 d, float end, Pcg32& rng,
+                               float& batch_end, unsigned ln, unsigned mask) {
+    const unsigned c = ln & 3u, base = ln & 28u;
+    bool occluded = false, stop = false;
+#pragma unroll 1
+    for (int r = 0; r < K / 4; ++r) {
+        float th;
+        unsigned id;
+        quad_hit(t, r, c, base, mask, th, id);
+        const bool hit = !stop && id != kNoHit && !(th > end);
+        float alpha = 0.0f;
+        if (hit && !self_occluded(P, th, id, d)) {
+            float dns;
+            const Response res = respond(P, id, o, d, dns);
+            alpha = (res.gres > P.min_response && res.alpha > P.alpha_min) ? res.alpha : 0.0f;
+        }
+        const unsigned hits = (__ballot_sync(mask, hit) >> base) & 15u;
+#pragma unroll
+        for (unsigned i = 0; i < 4; ++i) {
+            const float ai = __shfl_sync(mask, alpha, base + i), ti = __shfl_sync(mask, th, base + i);
+            if (stop || occluded) continue;
+            if (!((hits >> i) & 1u)) {
+                stop = true;
+                continue;
+            }
+            batch_end = fmaxf(batch_end, ti);
+            if (ai > 0.0f && rng.uniform() < ai) occluded = true;
+        }
+        stop = stop || occluded;
+        if (!__any_sync(mask, !stop)) break;
+    }
+    return occluded;
+}
+
 }  // namespace ptir

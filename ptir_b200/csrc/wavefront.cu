@@ -431,7 +431,7 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
 // Shared memory of a quad: its traversal stack (the staging of quad_composite lies over it: no traversal
 // is in progress then) and its compositing state.
 struct QuadSlot {
-    StackEntry stack[kStackDepth + kQuadStackPad];
+    StackEntry stack[kQuadStackEntries];
     QuadComposite comp;
 };
 static_assert(sizeof(float4) * kQuadStage <= sizeof(StackEntry) * kStackDepth, "the staging fits the stack");
@@ -658,12 +658,14 @@ __global__ void __launch_bounds__(kMaxThreads) k_wf_fwd_primary(TraceParams P, F
 // walk this cut the stage by 15 % on the 1M-Gaussian scene, and the register cap of the
 // intersection kernel (more resident warps) by 6 % more.
 template <int K>
-__global__ void __maxnreg__(trace_regs(K)) k_wf_shadow(TraceParams P, WfView W, int refill, const unsigned* items) {
+__global__ void __maxnreg__(trace_regs(K)) k_wf_shadow(TraceParams P, WfView W, int refill, const unsigned* items,
+                                                          unsigned quad_rays) {
     StackEntry stack[kStackDepth];
     TraceCounters ctr = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     constexpr unsigned kFull = 0xFFFFFFFFu;
     enum : int { kIdle = 0, kTracing = 1, kReady = 2 };
     const unsigned count = W.count[kQShadow];
+    if (count <= quad_rays) return;  // the quads' launch
     int phase = kIdle;
     unsigned q = 0;
     int rounds = 0;
@@ -789,6 +791,124 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_shadow(TraceParams P, WfView W, 
             phase = kIdle;
         }
         push(W.q[kQBounce], W.count + kQBounce, q, done);
+    }
+    flush_counters(P, ctr);
+}
+
+// k_wf_shadow for small launches, a quad of lanes a ray (quad.cuh): the same candidates, walked in the same order with
+// the same draws; no first round is seeded, as in k_wf_trace_quad. As there a small launch waits for its slowest
+// ray: stage of 16k rays over 10k Gaussians 0.60 -> 0.26 ms, of 90k over 300k (forward and adjoint) 6.6 -> 3.6 ms.
+template <int K>
+__global__ void __maxnreg__(96) k_wf_shadow_quad(TraceParams P, WfView W, int refill, const unsigned* items,
+                                                 unsigned quad_rays) {
+    extern __shared__ float4 quad_mem[];
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    enum : int { kIdle = 0, kTracing = 1, kReady = 2 };
+    const unsigned ln = lane(), c = ln & 3u, base = ln & 28u;
+    StackEntry* const stack = reinterpret_cast<StackEntry*>(quad_mem) + (threadIdx.x >> 2) * kQuadStackEntries;
+    TraceCounters ctr = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const unsigned count = W.count[kQShadow];
+    if (count > quad_rays) return;
+    const bool in_use = (ln >> 2) < quads_in_use(count);
+    int phase = kIdle;
+    unsigned q = 0;
+    int rounds = 0;
+    bool drained = false, seeded = false;
+    float3 ro = f3(0.0f), rd = f3(0.0f);
+    float start = 0.0f, end = 0.0f;
+    Pcg32 rng;
+    QuadTrace<K> t;
+    t.tk = kFarT;
+    kbuf_clear(t.kt, t.kid);
+    // next trace call of the quad's ray over (start, end); false when the ray is decided (unoccluded)
+    auto next_call = [&](float span) -> bool {
+        if (!(start < end)) return false;
+        if (++rounds > (1 << 16) + 1) {
+            if (c == 0) atomicOr(P.error_word, kErrLoopBound);
+            return false;
+        }
+        float cap = kFarT;
+        seeded = false;
+        if (K == 16 && span > 0.0f) {
+            cap = start + 1e-9f + kSeedSpan * span;
+            seeded = cap < end;
+            if (!seeded) cap = kFarT;
+        }
+        phase = quad_start(P.accel, ro, rd, start + 1e-9f, end, t, ctr, c, cap) ? kTracing : kReady;
+        return true;
+    };
+    while (true) {
+        bool done = false, occluded = false;
+        const unsigned idle = __ballot_sync(kFull, phase == kIdle && in_use && c == 0);
+        if (!drained && idle) {
+            const unsigned n_idle = __popc(idle);
+            unsigned first = 0;
+            if (ln == 0) first = atomicAdd(W.cursor + 3, n_idle);
+            first = __shfl_sync(kFull, first, 0);
+            drained = first + n_idle >= count;
+            const unsigned i = first + __popc(idle & ((1u << base) - 1u));
+            if (phase == kIdle && in_use && i < count) {
+                q = items[i];
+                const float3 wi = W.ps[q].em.dir;
+                ro = W.seg[q].pos + wi * 2e-2f;
+                rd = wi;
+                rng = load_rng(W, q);
+                if (c == 0) ++ctr.segments;
+                rounds = 0;
+                const float2 clip = clip_scene(P, ro, rd);
+                start = fmaxf(0.0f, clip.x - 1e-9f);
+                end = fminf(W.ps[q].em.tmax, clip.y) + 1e-9f;
+                phase = kTracing;
+                if (!next_call(0.0f)) done = true;  // nothing in front of the light
+            }
+        }
+        const unsigned busy = __ballot_sync(kFull, phase != kIdle && !done && c == 0);
+        if (!busy && !__any_sync(kFull, done)) {
+            if (drained) break;
+            continue;
+        }
+        // traverse until enough quads wait
+        while (true) {
+            const unsigned tracing = __ballot_sync(kFull, phase == kTracing && !done);
+            if (!tracing || __popc(busy) - (__popc(tracing) >> 2) >= (drained ? 1 : refill)) break;
+            if (phase == kTracing && !done && !quad_step<K, false>(P.accel, ro, rd, t, stack, P.error_word, ctr, ln, tracing)) {
+                if (seeded && t.tk >= kFarT) {
+                    seeded = false;
+                    quad_continue(t, ctr);
+                } else {
+                    phase = kReady;
+                }
+            }
+        }
+        // walk the finished batches: the first hit that occludes decides the ray
+        const bool ready = phase == kReady && !done;
+        const unsigned ready_m = __ballot_sync(kFull, ready);
+        if (ready) {
+            const float t_first = __shfl_sync(ready_m, t.kt[0], base);
+            const float t_last = __shfl_sync(ready_m, t.kt[QuadTrace<K>::L - 1], base + 3u);
+            float batch_end = start;
+            occluded = quad_shadow_walk(P, t, ro, rd, end, rng, batch_end, ln, ready_m);
+            if (occluded || batch_end <= start || !(t_last < kFarT)) {
+                done = true;  // decided, or no candidate left (the k-buffer was not full)
+            } else {
+                start = batch_end;
+                if (!next_call(t_last - t_first)) done = true;
+            }
+        }
+        if (done) {
+            if (c == 0) {
+                if (occluded) {
+                    Emitter em = W.ps[q].em;
+                    emitter_clear(em);
+                    W.ps[q].em = em;
+                }
+                if (P.flags & kPathSig) W.ps[q].sig = sig_mix(W.ps[q].sig, kSigShadow | (occluded ? 1u : 0u));
+                store_rng(W, q, rng);
+            }
+            phase = kIdle;
+        }
+        __syncwarp();
+        push(W.q[kQBounce], W.count + kQBounce, q, done && c == 0);
     }
     flush_counters(P, ctr);
 }
@@ -947,10 +1067,21 @@ int grid_cached(const void* fn, int block, size_t smem);
 // walk usually ends in its first batch, which a smaller buffer gathers with less traversal.
 static void launch_shadow(int ks, const TraceParams& q, const WfView& W, int B, int R, const unsigned* items,
                           cudaStream_t s) {
+    // up to kQuadRays shadow rays (the queue's count, which only the device knows) go to the quads
+    const auto blocks = [&](int grid, unsigned per_block) {
+        return (unsigned)std::min<long long>(grid, ((long long)W.slots + per_block - 1) / per_block);
+    };
+    const size_t stacks = sizeof(StackEntry) * kQuadStackEntries * (size_t)(B / 4);
+    const auto lanes = [&](auto* fn, unsigned quad_rays) {
+        if (W.slots > quad_rays) fn<<<blocks(grid_cached((const void*)fn, B, 0), B), B, 0, s>>>(q, W, R, items, quad_rays);
+    };
+    const auto quads = [&](auto* fn) {
+        fn<<<blocks(grid_cached((const void*)fn, B, stacks), B / 32), B, stacks, s>>>(q, W, (R + 3) / 4, items, kQuadRays);
+    };
     switch (ks) {
-    case 8: k_wf_shadow<8><<<grid_cached((const void*)k_wf_shadow<8>, B, 0), B, 0, s>>>(q, W, R, items); break;
-    case 32: k_wf_shadow<32><<<grid_cached((const void*)k_wf_shadow<32>, B, 0), B, 0, s>>>(q, W, R, items); break;
-    default: k_wf_shadow<16><<<grid_cached((const void*)k_wf_shadow<16>, B, 0), B, 0, s>>>(q, W, R, items); break;
+    case 8: quads(k_wf_shadow_quad<8>); lanes(k_wf_shadow<8>, kQuadRays); break;
+    case 32: lanes(k_wf_shadow<32>, 0u); break;
+    default: quads(k_wf_shadow_quad<16>); lanes(k_wf_shadow<16>, kQuadRays); break;
     }
 }
 
