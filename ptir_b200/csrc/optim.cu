@@ -11,18 +11,64 @@ namespace ptir {
 
 namespace {
 
-// one thread per 4 consecutive elements when the row length allows it, else per element
+// One element: the moments and the parameter of a visible row.
+__device__ __forceinline__ void adam_element(float g, float& p, float& m, float& v, float lr, float b1, float b2, float eps) {
+    const float mi = b1 * m + (1.0f - b1) * g;
+    const float vi = b2 * v + (1.0f - b2) * g * g;
+    p += __fdiv_rn(-lr * mi, __fadd_rn(__fsqrt_rn(vi), eps));
+    m = mi;
+    v = vi;
+}
+
+// One thread per four consecutive elements, read and written as 16 bytes each, whatever the row length: the four
+// may belong to two or more rows, and a hidden row's elements go back as they came. Nothing is read of a hidden
+// four but its rows' flags. Bound by HBM (28 bytes an element of a visible row); with one element a thread
+// a 64-bit division by the row length each stood before the loads: 300,000 rows of 48, 60 % of them visible, took
+// 80.2 us and take 56.7 (242 MB, 4.3 TB/s). Index: unsigned while the elements fit.
+template <class Index>
+__global__ void __launch_bounds__(256) k_selective_adam4(float4* __restrict__ param, const float4* __restrict__ grad,
+                                                         float4* __restrict__ m, float4* __restrict__ v,
+                                                         const uint8_t* __restrict__ visible, Index fours, Index row,
+                                                         float lr, float b1, float b2, float eps) {
+    const Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= fours) return;
+    bool on[4] = {true, true, true, true};
+    if (visible) {
+        const Index first = 4 * i;
+        Index r = first / row, left = (r + 1) * row - first;  // elements of row r from here on
+        bool f = visible[r] != 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (left == 0) {
+                f = visible[++r] != 0;
+                left = row;
+            }
+            on[k] = f;
+            --left;
+        }
+        if (!(on[0] || on[1] || on[2] || on[3])) return;
+    }
+    float4 p4 = param[i], m4 = m[i], v4 = v[i];
+    const float4 g4 = grad[i];
+    if (on[0]) adam_element(g4.x, p4.x, m4.x, v4.x, lr, b1, b2, eps);
+    if (on[1]) adam_element(g4.y, p4.y, m4.y, v4.y, lr, b1, b2, eps);
+    if (on[2]) adam_element(g4.z, p4.z, m4.z, v4.z, lr, b1, b2, eps);
+    if (on[3]) adam_element(g4.w, p4.w, m4.w, v4.w, lr, b1, b2, eps);
+    param[i] = p4;
+    m[i] = m4;
+    v[i] = v4;
+}
+
+// one element per thread: the elements after the last four, and buffers that are not 16-byte aligned
 __global__ void k_selective_adam(float* __restrict__ param, const float* __restrict__ grad, float* __restrict__ m,
-                                 float* __restrict__ v, const uint8_t* __restrict__ visible, long long n_rows,
-                                 int row, float lr, float b1, float b2, float eps) {
-    const long long total = n_rows * (long long)row;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+                                 float* __restrict__ v, const uint8_t* __restrict__ visible, long long first,
+                                 long long total, int row, float lr, float b1, float b2, float eps) {
+    for (long long i = first + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
         if (visible && !visible[i / row]) continue;
-        const float g = grad[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * g;
-        const float vi = b2 * v[i] + (1.0f - b2) * g * g;
-        param[i] += __fdiv_rn(-lr * mi, __fadd_rn(__fsqrt_rn(vi), eps));
+        float p = param[i], mi = m[i], vi = v[i];
+        adam_element(grad[i], p, mi, vi, lr, b1, b2, eps);
+        param[i] = p;
         m[i] = mi;
         v[i] = vi;
     }
@@ -52,10 +98,28 @@ extern "C" int ptir_selective_adam(float* param, const float* grad, float* exp_a
     if (n_rows == 0) return PTIR_OK;
     if (!param || !grad || !exp_avg || !exp_avg_sq) return PTIR_EINVAL;
     const long long total = n_rows * (long long)row;
+    const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int block = 256;
-    const long long blocks = (total + block - 1) / block;
-    const unsigned grid = (unsigned)(blocks < 148LL * 64 ? blocks : 148LL * 64);
-    ptir::k_selective_adam<<<grid, block, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        param, grad, exp_avg, exp_avg_sq, visible, n_rows, row, lr, beta1, beta2, eps);
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(param) | reinterpret_cast<uintptr_t>(grad) |
+                           reinterpret_cast<uintptr_t>(exp_avg) | reinterpret_cast<uintptr_t>(exp_avg_sq);
+    const long long fours = (bits & 15u) == 0 ? total / 4 : 0, tail = total - 4 * fours;
+    if (fours > 0) {
+        const long long grid = (fours + block - 1) / block;
+        if (grid > 0x7FFFFFFFll) return PTIR_EINVAL;
+        const auto as4 = [](float* p) { return reinterpret_cast<float4*>(p); };
+        const float4* g4 = reinterpret_cast<const float4*>(grad);
+        if (total + row < (1ll << 31))
+            ptir::k_selective_adam4<unsigned><<<(unsigned)grid, block, 0, s>>>(
+                as4(param), g4, as4(exp_avg), as4(exp_avg_sq), visible, (unsigned)fours, (unsigned)row, lr, beta1, beta2, eps);
+        else
+            ptir::k_selective_adam4<long long><<<(unsigned)grid, block, 0, s>>>(
+                as4(param), g4, as4(exp_avg), as4(exp_avg_sq), visible, fours, (long long)row, lr, beta1, beta2, eps);
+    }
+    if (tail > 0) {
+        const long long blocks = (tail + block - 1) / block;
+        const unsigned grid = (unsigned)(blocks < 148LL * 64 ? blocks : 148LL * 64);
+        ptir::k_selective_adam<<<grid, block, 0, s>>>(param, grad, exp_avg, exp_avg_sq, visible, 4 * fours, total, row, lr,
+                                                      beta1, beta2, eps);
+    }
     return cudaGetLastError() == cudaSuccess ? PTIR_OK : PTIR_ECUDA;
 }
