@@ -19,6 +19,9 @@ class SelectiveAdam(torch.optim.Adam):
 
     @torch.no_grad()
     def step(self, visibility):
+        # the flags of the first n rows, one byte each, made once for all groups of n rows (a step of a small or
+        # medium scene is bound by the host, not by the kernel)
+        flags, streams = {}, {}
         for group in self.param_groups:
             lr, eps = group["lr"], group["eps"]
             beta1, beta2 = group["betas"]
@@ -40,11 +43,16 @@ class SelectiveAdam(torch.optim.Adam):
             row = param.numel() // max(n, 1)
             vis = None
             if visibility is not None:
-                vis = (visibility.reshape(-1)[:n] != 0).to(device=param.device, dtype=torch.uint8).contiguous()
+                vis = flags.get((n, param.device))
+                if vis is None:
+                    vis = flags[n, param.device] = (visibility.reshape(-1)[:n] != 0).to(device=param.device)
+            stream = streams.get(param.device)
+            if stream is None:
+                stream = streams[param.device] = torch.cuda.current_stream(param.device).cuda_stream
             rc = self._lib.ptir_selective_adam(
                 param.data_ptr(), grad.data_ptr(), state["exp_avg"].data_ptr(), state["exp_avg_sq"].data_ptr(),
                 None if vis is None else vis.data_ptr(), int(n), int(max(row, 1)), float(lr), float(beta1),
-                float(beta2), float(eps), torch.cuda.current_stream(param.device).cuda_stream)
+                float(beta2), float(eps), stream)
             if rc != N.PTIR_OK:
                 raise N.PtirError(rc, "ptir_selective_adam failed")
 
