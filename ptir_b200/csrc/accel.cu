@@ -235,6 +235,8 @@ constexpr int kPlocRadius = 16;
 constexpr int kPlocThreads = 256;
 constexpr int kPlocScanThreads = 1024;
 constexpr int kPlocBatch = 4;  // iterations launched between reads of the cluster count
+constexpr int kPlocTail = 3072;  // clusters from which one block finishes the list (k_ploc_tail)
+constexpr int kPlocTailThreads = 1024;
 
 // surface area (halved) of the union of two boxes; the same value whichever box comes first
 __device__ __forceinline__ float ploc_area(float4 alo, float4 ahi, float4 blo, float4 bhi) {
@@ -411,6 +413,146 @@ __global__ void __launch_bounds__(kPlocThreads) k_ploc_compact(const unsigned* _
     }
 }
 
+// A pair's place in the order of the pairs (area, list distance, parity of the lower index, lower index) as the
+// neighbour search of k_ploc_nn ranks them.
+struct PlocPair {
+    float area;
+    int dist, lower, other;  // other: the neighbour, -1 none
+};
+__device__ __forceinline__ bool ploc_before(const PlocPair& a, const PlocPair& b) {
+    if (a.other < 0 || b.other < 0) return a.other >= 0;
+    if (a.area != b.area) return a.area < b.area;
+    if (a.dist != b.dist) return a.dist < b.dist;
+    if ((a.lower & 1) != (b.lower & 1)) return (a.lower & 1) < (b.lower & 1);
+    return a.lower < b.lower;
+}
+
+// The iterations from kPlocTail clusters to the root, in one block with the list in shared memory. Most of a build's
+// iterations are here: the last few thousand clusters merge a few pairs at a time (a million Gaussians take about
+// 16 iterations to 3000 clusters and 110 from there), and as launches each cost four kernels of a few us and a
+// quarter of a host round trip. As many lanes as fit share the search of a cluster's 32 neighbours; the
+// order of pairs is strict, so the pairs are those of k_ploc_nn and k_ploc_merge. Bound by the latency of the
+// iteration (search, merge, scan): a rebuild of a million Gaussians took 10.75 ms and takes TIMED with this kernel,
+// the collapse in parallel (k_collapse_level) and the scratch kept.
+struct PlocTail {
+    float box[2][6][kPlocTail];
+    int cid[2][kPlocTail];
+    int nn[kPlocTail];
+    unsigned wsum[32];
+    int next_node;
+};
+
+static_assert(sizeof(PlocTail) <= 227 * 1024, "shared memory of a block");
+
+__global__ void __launch_bounds__(kPlocTailThreads) k_ploc_tail(int n, const unsigned* __restrict__ count_p,
+                                                                const int* __restrict__ cid_in,
+                                                                const float4* __restrict__ cb_in,
+                                                                float4* __restrict__ nodes, int* __restrict__ parent,
+                                                                unsigned* next_node) {
+    extern __shared__ __align__(16) unsigned char ploc_mem[];
+    PlocTail& T = *reinterpret_cast<PlocTail*>(ploc_mem);
+    int count = min((int)*count_p, kPlocTail);
+    const int tid = (int)threadIdx.x;
+    for (int i = tid; i < count; i += kPlocTailThreads) {
+        const float4 lo = cb_in[2 * (size_t)i], hi = cb_in[2 * (size_t)i + 1];
+        T.box[0][0][i] = lo.x; T.box[0][1][i] = lo.y; T.box[0][2][i] = lo.z;
+        T.box[0][3][i] = hi.x; T.box[0][4][i] = hi.y; T.box[0][5][i] = hi.z;
+        T.cid[0][i] = cid_in[i];
+    }
+    if (tid == 0) T.next_node = (int)*next_node;
+    __syncthreads();
+    int cur = 0;
+    // every iteration merges at least one pair
+    for (int guard = 0; count > 1 && guard < kPlocTail; ++guard) {
+        const float(*box)[kPlocTail] = T.box[cur];
+        // lanes to a cluster: a power of two up to 32
+        int group = 1;
+        while (group < 32 && 2 * group * count <= kPlocTailThreads) group *= 2;
+        const int sub = tid & (group - 1);
+        for (int base = 0; base < count; base += kPlocTailThreads / group) {
+            const int i = base + tid / group;
+            PlocPair best{INFINITY, 0, 0, -1};
+            if (i < count) {
+                const float4 lo = make_float4(box[0][i], box[1][i], box[2][i], 0.0f);
+                const float4 hi = make_float4(box[3][i], box[4][i], box[5][i], 0.0f);
+                for (int k = sub; k < 2 * kPlocRadius; k += group) {
+                    const int j = i + (k < kPlocRadius ? k - kPlocRadius : k - kPlocRadius + 1);
+                    if (j < 0 || j >= count) continue;
+                    PlocPair p;
+                    p.area = ploc_area(lo, hi, make_float4(box[0][j], box[1][j], box[2][j], 0.0f),
+                                       make_float4(box[3][j], box[4][j], box[5][j], 0.0f));
+                    p.dist = j < i ? i - j : j - i;
+                    p.lower = min(i, j);
+                    p.other = j;
+                    if (ploc_before(p, best)) best = p;
+                }
+            }
+            for (int o = group / 2; o > 0; o >>= 1) {
+                PlocPair p;
+                p.area = __shfl_xor_sync(0xFFFFFFFFu, best.area, o);
+                p.dist = __shfl_xor_sync(0xFFFFFFFFu, best.dist, o);
+                p.lower = __shfl_xor_sync(0xFFFFFFFFu, best.lower, o);
+                p.other = __shfl_xor_sync(0xFFFFFFFFu, best.other, o);
+                if (ploc_before(p, best)) best = p;
+            }
+            if (i < count && sub == 0) T.nn[i] = best.other;
+        }
+        __syncthreads();
+        // merge mutual neighbours into the left one's place and compact, four consecutive clusters a thread
+        const int per = (count + kPlocTailThreads - 1) / kPlocTailThreads;
+        const int first = min(count, tid * per), last = min(count, first + per);
+        unsigned kept = 0;
+        for (int i = first; i < last; ++i) {
+            const int j = T.nn[i];
+            kept += (j >= 0 && j < i && T.nn[j] == i) ? 0u : 1u;
+        }
+        unsigned inc = kept;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if ((tid & 31) >= o) inc += y;
+        }
+        if ((tid & 31) == 31) T.wsum[tid >> 5] = inc;
+        __syncthreads();
+        if (tid < 32) {
+            unsigned x = T.wsum[tid];
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (tid >= o) x += y;
+            }
+            T.wsum[tid] = x;
+        }
+        __syncthreads();
+        unsigned at = inc - kept + (tid >= 32 ? T.wsum[(tid >> 5) - 1] : 0u);
+        for (int i = first; i < last; ++i) {
+            const int j = T.nn[i];
+            const bool mutual = j >= 0 && T.nn[j] == i;
+            if (mutual && j < i) continue;
+            int id = T.cid[cur][i];
+            float b[6];
+            for (int k = 0; k < 6; ++k) b[k] = T.box[cur][k][i];
+            if (mutual) {
+                const int idx = atomicSub(&T.next_node, 1) - 1, r = T.cid[cur][j];
+                nodes[4 * (size_t)idx + 3] = make_float4(__int_as_float(id), __int_as_float(r), 0.0f, 0.0f);
+                parent[id < 0 ? (n - 1) + ~id : id] = idx;
+                parent[r < 0 ? (n - 1) + ~r : r] = idx;
+                for (int k = 0; k < 3; ++k) b[k] = fminf(b[k], T.box[cur][k][j]);
+                for (int k = 3; k < 6; ++k) b[k] = fmaxf(b[k], T.box[cur][k][j]);
+                id = idx;
+            }
+            T.cid[1 - cur][at] = id;
+            for (int k = 0; k < 6; ++k) T.box[1 - cur][k][at] = b[k];
+            ++at;
+        }
+        count = (int)T.wsum[31];
+        cur = 1 - cur;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        *next_node = (unsigned)T.next_node;
+        parent[0] = -1;  // the root
+    }
+}
+
 // box and kmax of child c of the hierarchy
 __device__ __forceinline__ void child_box(const float4* __restrict__ sbox_unsorted, const unsigned* __restrict__ order,
                                           const float4* nodes, int c, float3& lo, float3& hi, float& kmax) {
@@ -459,9 +601,16 @@ __global__ void k_refit(int n, const float4* __restrict__ box, const unsigned* _
 // become the roots of further 4-wide nodes. Against taking every binary node at even depth with its
 // grandchildren, this fills nodes whose children include leaves; a simulation of the tracer's
 // traversal on the 1M-Gaussian scene (camera rays, k-buffer 16) measured 11 % fewer node visits.
-// One block, level by level: wide node w has binary root wroot[w]; its children are recorded as
-// binary references (wsrc, for refits) and as wide-node indices or leaves (wchild).
+// Wide node w has binary root wroot[w]; its children are recorded as binary references (wsrc, for refits) and
+// as wide-node indices or leaves (wchild). Level by level: the first levels, and whatever is left after
+// kCollapseLevels launches, by one block; the wide levels between by as many as there are nodes for (one block for
+// all 461,000 wide nodes of a million Gaussians took 2.35 ms).
 constexpr int kCollapseThreads = 1024;
+constexpr int kCollapseLevels = 24;
+constexpr unsigned kCollapseWide = 512;  // nodes of a level from which more blocks than one take it
+
+// counters of the collapse: wide nodes handed out (the count at the end), the level's range, finished blocks
+enum : int { kWideTail = 0, kWideHead = 1, kWideEnd = 2, kWideTicket = 3, kWideCounters = 4 };
 
 __device__ __forceinline__ float box_area(float3 lo, float3 hi) {
     const float3 e = hi - lo;
@@ -482,67 +631,138 @@ __device__ __forceinline__ void record_child(const float4* nd, int side, int& c,
     }
 }
 
-__global__ void __launch_bounds__(kCollapseThreads) k_collapse4(int n, const float4* __restrict__ nodes,
-                                                                int* __restrict__ wroot, int* __restrict__ wsrc,
-                                                                int* __restrict__ wchild, unsigned* __restrict__ wcount) {
-    __shared__ unsigned tail;
+// Wide node w (when `live`; called by whole warps): its children, the internal ones given the next indices, those of
+// one node together.
+__device__ void collapse_node(bool live, unsigned w, const float4* __restrict__ nodes, int* __restrict__ wroot,
+                              int* __restrict__ wsrc, int* __restrict__ wchild, unsigned* tail) {
+    int ref[4] = {kNoChild, kNoChild, kNoChild, kNoChild};
+    int cnt = 0;
+    if (live) {
+        float area[4];
+        cnt = 2;
+        const float4* nb = nodes + 4 * (size_t)wroot[w];
+        for (int side = 0; side < 2; ++side) {
+            float3 lo, hi;
+            record_child(nb, side, ref[side], lo, hi);
+            area[side] = box_area(lo, hi);
+        }
+        while (cnt < 4) {
+            int best = -1;
+            float barea = -1.0f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < cnt && ref[k] >= 0 && area[k] > barea) {
+                    barea = area[k];
+                    best = k;
+                }
+            if (best < 0) break;
+            int from = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k == best) from = ref[k];
+            const float4* nc = nodes + 4 * (size_t)from;
+            float3 llo, lhi, rlo, rhi;
+            int l, r;
+            record_child(nc, 0, l, llo, lhi);
+            record_child(nc, 1, r, rlo, rhi);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (k == best) {
+                    ref[k] = l;
+                    area[k] = box_area(llo, lhi);
+                } else if (k == cnt) {
+                    ref[k] = r;
+                    area[k] = box_area(rlo, rhi);
+                }
+            }
+            ++cnt;
+        }
+    }
+    unsigned inner = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) inner += (k < cnt && ref[k] >= 0) ? 1u : 0u;
+    unsigned inc = inner;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if ((threadIdx.x & 31u) >= (unsigned)o) inc += y;
+    }
+    unsigned base = 0;
+    if ((threadIdx.x & 31u) == 31u && inc) base = atomicAdd(tail, inc);
+    base = __shfl_sync(0xFFFFFFFFu, base, 31);
+    if (!live) return;
+    unsigned idx = base + inc - inner;
+    int link[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        link[k] = k < cnt ? ref[k] : kNoChild;
+        if (k < cnt && ref[k] >= 0) {
+            wroot[idx] = ref[k];
+            link[k] = (int)idx++;
+        }
+    }
+    reinterpret_cast<int4*>(wsrc)[w] = make_int4(ref[0], ref[1], ref[2], ref[3]);
+    reinterpret_cast<int4*>(wchild)[w] = make_int4(link[0], link[1], link[2], link[3]);
+}
+
+// One block: the levels from the current one on while they hold less than `wide` nodes (0xFFFFFFFF: to the end). The
+// first launch starts at the root. Every wide node takes at least one binary node, so the loop ends after at most
+// n - 1 levels.
+__global__ void __launch_bounds__(kCollapseThreads) k_collapse_block(int n, const float4* __restrict__ nodes,
+                                                                     int* __restrict__ wroot, int* __restrict__ wsrc,
+                                                                     int* __restrict__ wchild, unsigned* __restrict__ ctr,
+                                                                     bool first, unsigned wide) {
+    __shared__ unsigned head, end;
     if (threadIdx.x == 0) {
-        tail = 1u;
-        wroot[0] = 0;
+        if (first) {
+            wroot[0] = 0;
+            ctr[kWideTail] = 1u;
+            ctr[kWideTicket] = 0u;
+            head = 0u;
+            end = 1u;
+        } else {
+            head = ctr[kWideHead];
+            end = ctr[kWideEnd];
+        }
+        __threadfence();
     }
     __syncthreads();
-    unsigned head = 0;
-    // every wave consumes at least one wide node and each binary node roots at most one, so the
-    // loop ends after at most n - 1 waves
-    for (int wave = 0; wave < n; ++wave) {
-        const unsigned end = tail;
+    for (int level = 0; level < n && head < end && end - head < wide; ++level) {
+        const unsigned a = head, b = end;
+        for (unsigned w0 = a; w0 < b; w0 += kCollapseThreads) {
+            const unsigned w = w0 + threadIdx.x;
+            collapse_node(w < b, w, nodes, wroot, wsrc, wchild, ctr + kWideTail);
+        }
+        __threadfence();
         __syncthreads();
-        for (unsigned w = head + threadIdx.x; w < end; w += blockDim.x) {
-            int ref[4];
-            float area[4];
-            int cnt = 2;
-            const float4* nb = nodes + 4 * (size_t)wroot[w];
-            for (int side = 0; side < 2; ++side) {
-                float3 lo, hi;
-                record_child(nb, side, ref[side], lo, hi);
-                area[side] = box_area(lo, hi);
-            }
-            while (cnt < 4) {
-                int best = -1;
-                float barea = -1.0f;
-                for (int k = 0; k < cnt; ++k)
-                    if (ref[k] >= 0 && area[k] > barea) {
-                        barea = area[k];
-                        best = k;
-                    }
-                if (best < 0) break;
-                const float4* nc = nodes + 4 * (size_t)ref[best];
-                float3 lo, hi;
-                record_child(nc, 0, ref[best], lo, hi);
-                area[best] = box_area(lo, hi);
-                record_child(nc, 1, ref[cnt], lo, hi);
-                area[cnt] = box_area(lo, hi);
-                ++cnt;
-            }
-            for (int k = 0; k < 4; ++k) {
-                int src = kNoChild, link = kNoChild;
-                if (k < cnt) {
-                    src = link = ref[k];
-                    if (ref[k] >= 0) {
-                        const unsigned idx = atomicAdd(&tail, 1u);
-                        wroot[idx] = ref[k];
-                        link = (int)idx;
-                    }
-                }
-                wsrc[4 * (size_t)w + k] = src;
-                wchild[4 * (size_t)w + k] = link;
-            }
+        if (threadIdx.x == 0) {
+            head = b;
+            end = atomicAdd(ctr + kWideTail, 0u);
         }
         __syncthreads();
-        head = end;
-        if (head == tail) break;
     }
-    if (threadIdx.x == 0) *wcount = tail;
+    if (threadIdx.x == 0) {
+        ctr[kWideHead] = head;
+        ctr[kWideEnd] = end;
+    }
+}
+
+// One level by the whole grid; the last block to finish opens the next.
+__global__ void __launch_bounds__(256) k_collapse_level(const float4* __restrict__ nodes, int* __restrict__ wroot,
+                                                        int* __restrict__ wsrc, int* __restrict__ wchild,
+                                                        unsigned* __restrict__ ctr) {
+    const unsigned a = ctr[kWideHead], b = ctr[kWideEnd];
+    if (a >= b) return;
+    for (unsigned w0 = a + blockIdx.x * blockDim.x; w0 < b; w0 += gridDim.x * blockDim.x) {
+        const unsigned w = w0 + threadIdx.x;
+        collapse_node(w < b, w, nodes, wroot, wsrc, wchild, ctr + kWideTail);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(ctr + kWideTicket, 1u) == gridDim.x - 1u) {
+        ctr[kWideTicket] = 0u;
+        ctr[kWideHead] = b;
+        ctr[kWideEnd] = atomicAdd(ctr + kWideTail, 0u);
+    }
 }
 
 // 4-wide node w: the boxes of its children (binary references wsrc, from the refitted binary
@@ -594,10 +814,16 @@ cudaError_t grow(T*& ptr, size_t count, cudaStream_t s) {
     return cudaMallocAsync(reinterpret_cast<void**>(&ptr), count * sizeof(T), s);
 }
 
-// The binary nodes and parent links of a PLOC build over the n > 1 leaves in key order
-// (st.ids[1]). Its scratch lives for the build only. Iterations are launched kPlocBatch at a
-// time, then the cluster count is read back; at most n - 1 iterations are needed, since each
-// merges at least one pair.
+// Bytes of a PLOC build's scratch: cluster boxes [2][2n] float4, cluster ids [2][n], neighbours [n], block counts,
+// counters [4].
+size_t ploc_scratch_bytes(size_t n) {
+    return 64 * n + (3 * n + (n + kPlocThreads - 1) / kPlocThreads + 4) * sizeof(int);
+}
+
+// The binary nodes and parent links of a PLOC build over the n > 1 leaves in key order (st.ids[1]), the root
+// without a parent. Its scratch lies in the 4-wide nodes (st.quads), which are written after it. Iterations are
+// launched until the list is down to kPlocTail clusters, the count read back every few of them, and one
+// block does the rest; at most n - 1 iterations are needed, since each merges at least one pair.
 cudaError_t ploc_build(AccelState& st, int n, cudaStream_t s, std::string& err) {
     cudaError_t e = cudaSuccess;
     if (!st.ploc_host) {
@@ -606,17 +832,16 @@ cudaError_t ploc_build(AccelState& st, int n, cudaStream_t s, std::string& err) 
             err = std::string("cudaMallocHost: ") + cudaGetErrorString(e);
             return e;
         }
+        // more than 48 KB of dynamic shared memory needs the kernel's opt-in (per device: with the state's buffers)
+        e = cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PlocTail));
+        if (e != cudaSuccess) {
+            err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
+            return e;
+        }
     }
     const int nb = (n + kPlocThreads - 1) / kPlocThreads;
-    // cluster boxes [2][2n] float4, cluster ids [2][n], neighbours [n], block counts [nb], counters [4]
     const size_t box_bytes = 2 * sizeof(float4) * (size_t)n;
-    const size_t bytes = 2 * box_bytes + (3 * (size_t)n + (size_t)nb + 4) * sizeof(int) + 256;
-    char* scratch = nullptr;
-    e = cudaMallocAsync(reinterpret_cast<void**>(&scratch), bytes, s);
-    if (e != cudaSuccess) {
-        err = std::string("cudaMallocAsync (PLOC scratch): ") + cudaGetErrorString(e);
-        return e;
-    }
+    char* scratch = reinterpret_cast<char*>(st.quads);
     float4* cb[2] = {reinterpret_cast<float4*>(scratch), reinterpret_cast<float4*>(scratch + box_bytes)};
     int* cid[2] = {reinterpret_cast<int*>(scratch + 2 * box_bytes), reinterpret_cast<int*>(scratch + 2 * box_bytes) + n};
     int* nn = cid[1] + n;
@@ -626,46 +851,47 @@ cudaError_t ploc_build(AccelState& st, int n, cudaStream_t s, std::string& err) 
     k_ploc_init<<<nb, kPlocThreads, 0, s>>>(n, st.box, st.ids[1], cid[0], cb[0], cnt, next_node);
     e = cudaGetLastError();
     int cur = 0;
-    for (long long it = 0; e == cudaSuccess;) {
-        for (int b = 0; b < kPlocBatch; ++b, ++it) {
-            k_ploc_nn<<<nb, kPlocThreads, 0, s>>>(cnt + cur, cb[cur], nn);
-            k_ploc_merge<<<nb, kPlocThreads, 0, s>>>(n, cnt + cur, nn, cid[cur], cb[cur], st.nodes, st.parent, next_node,
-                                                     blk);
+    long long left = n;
+    // an iteration merges about a third of the clusters: the first read comes when the list might be short
+    int batch = 0;
+    for (double c = n; c > kPlocTail; c *= 0.66) ++batch;
+    for (long long it = 0; e == cudaSuccess && left > kPlocTail; batch = kPlocBatch) {
+        const unsigned blocks = (unsigned)((left + kPlocThreads - 1) / kPlocThreads);
+        for (int b = 0; b < batch; ++b, ++it) {
+            k_ploc_nn<<<blocks, kPlocThreads, 0, s>>>(cnt + cur, cb[cur], nn);
+            k_ploc_merge<<<blocks, kPlocThreads, 0, s>>>(n, cnt + cur, nn, cid[cur], cb[cur], st.nodes, st.parent,
+                                                         next_node, blk);
             k_ploc_scan<<<1, kPlocScanThreads, 0, s>>>(cnt + cur, blk, cnt + 1 - cur);
-            k_ploc_compact<<<nb, kPlocThreads, 0, s>>>(cnt + cur, nn, cid[cur], cb[cur], blk, cid[1 - cur], cb[1 - cur]);
+            k_ploc_compact<<<blocks, kPlocThreads, 0, s>>>(cnt + cur, nn, cid[cur], cb[cur], blk, cid[1 - cur], cb[1 - cur]);
             cur = 1 - cur;
         }
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(st.ploc_host, cnt + cur, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(st.ploc_host + 1, next_node, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            err = std::string("PLOC iteration: ") + cudaGetErrorString(e);
-            break;
-        }
-        if (st.ploc_host[0] <= 1u) {
-            if (st.ploc_host[1] != 0u) {  // n - 1 merges hand out every node index
-                err = "PLOC ended with " + std::to_string(st.ploc_host[1]) + " node indices unused";
-                e = cudaErrorUnknown;
-            }
-            break;
-        }
+        if (e != cudaSuccess) break;
+        left = (long long)st.ploc_host[0];
         if (it > (long long)n + kPlocBatch) {
             err = "PLOC did not converge";
-            e = cudaErrorUnknown;
-            break;
+            return cudaErrorUnknown;
         }
     }
     if (e == cudaSuccess) {
-        e = cudaMemsetAsync(st.parent, 0xFF, sizeof(int), s);  // the root (node 0) has no parent
-        if (e != cudaSuccess) err = std::string("cudaMemsetAsync: ") + cudaGetErrorString(e);
+        k_ploc_tail<<<1, kPlocTailThreads, sizeof(PlocTail), s>>>(n, cnt + cur, cid[cur], cb[cur], st.nodes, st.parent,
+                                                                  next_node);
+        e = cudaGetLastError();
     }
-    const cudaError_t f = cudaFreeAsync(scratch, s);
-    if (e == cudaSuccess && f != cudaSuccess) {
-        err = std::string("cudaFreeAsync (PLOC scratch): ") + cudaGetErrorString(f);
-        e = f;
+    // n - 1 merges hand out every node index
+    if (e == cudaSuccess) e = cudaMemcpyAsync(st.ploc_host + 1, next_node, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        err = std::string("PLOC iteration: ") + cudaGetErrorString(e);
+        return e;
     }
-    return e;
+    if (st.ploc_host[1] != 0u) {
+        err = "PLOC ended with " + std::to_string(st.ploc_host[1]) + " node indices unused";
+        return cudaErrorUnknown;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace
@@ -719,9 +945,9 @@ cudaError_t accel_build(AccelState& st, const AccelBuildOptions& opt, const floa
         PTIR_TRY(grow(st.wroot, cap, s));
         PTIR_TRY(grow(st.wsrc, 4 * cap, s));
         PTIR_TRY(grow(st.wchild, 4 * cap, s));
-        if (!st.wcount) PTIR_TRY(cudaMallocAsync(reinterpret_cast<void**>(&st.wcount), sizeof(unsigned), s));
+        if (!st.wcount) PTIR_TRY(cudaMallocAsync(reinterpret_cast<void**>(&st.wcount), kWideCounters * sizeof(unsigned), s));
         PTIR_TRY(grow(st.nodes4, 8 * (cap > 1 ? cap - 1 : 1), s));
-        PTIR_TRY(grow(st.quads, 8 * (cap > 1 ? cap - 1 : 1), s));
+        PTIR_TRY(grow(st.quads, std::max(8 * (cap > 1 ? cap - 1 : 1), ploc_scratch_bytes(cap) / sizeof(float4) + 1), s));
         st.capacity = cap;
         st.valid = false;
     }
@@ -766,7 +992,15 @@ cudaError_t accel_build(AccelState& st, const AccelBuildOptions& opt, const floa
         PTIR_TRY(cudaGetLastError());
         if (!refit) {
             // the 4-wide topology (kept by refits)
-            k_collapse4<<<1, kCollapseThreads, 0, s>>>(n, st.nodes, st.wroot, st.wsrc, st.wchild, st.wcount);
+            k_collapse_block<<<1, kCollapseThreads, 0, s>>>(n, st.nodes, st.wroot, st.wsrc, st.wchild, st.wcount, true,
+                                                            n > 4 * (int)kCollapseWide ? kCollapseWide : 0xFFFFFFFFu);
+            if (n > 4 * (int)kCollapseWide) {
+                const unsigned level_blocks = std::min(4u * 148u, blocks);
+                for (int level = 0; level < kCollapseLevels; ++level)
+                    k_collapse_level<<<level_blocks, T, 0, s>>>(st.nodes, st.wroot, st.wsrc, st.wchild, st.wcount);
+                k_collapse_block<<<1, kCollapseThreads, 0, s>>>(n, st.nodes, st.wroot, st.wsrc, st.wchild, st.wcount, false,
+                                                                0xFFFFFFFFu);
+            }
             PTIR_TRY(cudaGetLastError());
         }
         k_emit4<<<(unsigned)((n - 1 + T - 1) / T), T, 0, s>>>(n, st.nodes, st.box, st.ids[1], st.wsrc, st.wchild,
