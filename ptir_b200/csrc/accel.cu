@@ -233,7 +233,6 @@ __global__ void k_hierarchy(int n, const unsigned long long* __restrict__ keys, 
 // collapse and emit.
 constexpr int kPlocRadius = 16;
 constexpr int kPlocThreads = 256;
-constexpr int kPlocScanThreads = 1024;
 constexpr int kPlocBatch = 4;  // iterations launched between reads of the cluster count
 constexpr int kPlocTail = 3072;  // clusters from which one block finishes the list (k_ploc_tail)
 constexpr int kPlocTailThreads = 1024;
@@ -263,158 +262,126 @@ __global__ void k_ploc_init(int n, const float4* __restrict__ box, const unsigne
     cb[2 * (size_t)i + 1] = box[2 * (size_t)g + 1];
 }
 
-// nearest neighbour of every cluster within kPlocRadius positions (-1 when alone)
-__global__ void __launch_bounds__(kPlocThreads) k_ploc_nn(const unsigned* __restrict__ count_p,
-                                                          const float4* __restrict__ cb, int* __restrict__ nn) {
-    constexpr int kSpan = kPlocThreads + 2 * kPlocRadius;
+// An iteration is two launches. k_ploc_pair finds every cluster's nearest neighbour within kPlocRadius positions and
+// from it the cluster's partner (its neighbour when each is the other's, else -1), and counts per block the clusters
+// that stay in the list (all but the right one of each pair). k_ploc_merge writes the next list: it sums the
+// blocks before its own, puts a new binary node with its parent links in the left one's place, and the last block
+// hands on the count. (Neighbours, merge, scan of the block counts and compaction as a launch each took 37 us
+// an iteration over the 70 iterations from a million Gaussians to kPlocTail clusters; this takes 25.)
+//
+// A block finds the neighbours of its clusters and of the kPlocRadius on either side, which its own may pair with,
+// from the boxes of as many more around those.
+constexpr int kPlocPairThreads = kPlocThreads + 2 * kPlocRadius;
+
+__global__ void __launch_bounds__(kPlocPairThreads) k_ploc_pair(const unsigned* __restrict__ count_p,
+                                                                const float4* __restrict__ cb, int* __restrict__ partner,
+                                                                unsigned* __restrict__ blk) {
+    constexpr int kSpan = kPlocPairThreads + 2 * kPlocRadius;
     __shared__ float4 slo[kSpan], shi[kSpan];
+    __shared__ int nn[kPlocPairThreads];
+    __shared__ unsigned kept;
     const int count = (int)*count_p;
     const int b0 = blockIdx.x * kPlocThreads;
     if (b0 >= count) return;
-    for (int k = threadIdx.x; k < kSpan; k += kPlocThreads) {
-        const int j = b0 - kPlocRadius + k;
+    if (threadIdx.x == 0) kept = 0u;
+    for (int k = threadIdx.x; k < kSpan; k += kPlocPairThreads) {
+        const int j = b0 - 2 * kPlocRadius + k;
         if (j >= 0 && j < count) {
             slo[k] = cb[2 * (size_t)j];
             shi[k] = cb[2 * (size_t)j + 1];
         }
     }
     __syncthreads();
-    const int i = b0 + threadIdx.x;
-    if (i >= count) return;
-    const int s = threadIdx.x + kPlocRadius;
-    const float4 lo = slo[s], hi = shi[s];
-    int best = -1, bdist = 0, bmin = 0;
-    float barea = INFINITY;
-    for (int d = -kPlocRadius; d <= kPlocRadius; ++d) {
-        const int j = i + d;
-        if (d == 0 || j < 0 || j >= count) continue;
-        const float a = ploc_area(lo, hi, slo[s + d], shi[s + d]);
-        const int dist = d < 0 ? -d : d, mn = min(i, j);
-        // pairs ordered by (area, list distance, parity of the lower index, lower index): equal
-        // boxes (coincident Gaussians) then pair up as (0,1), (2,3), ... and halve every
-        // iteration, where the smaller index alone would merge one pair an iteration
-        const bool better = best < 0 || a < barea ||
-                            (a == barea && (dist < bdist || (dist == bdist && ((mn & 1) < (bmin & 1) ||
-                                                                               ((mn & 1) == (bmin & 1) && mn < bmin)))));
-        if (better) {
-            barea = a;
-            best = j;
-            bdist = dist;
-            bmin = mn;
-        }
-    }
-    nn[i] = best;
-}
-
-// number of clusters of a block that stay in the list (all but the right one of each merged pair)
-__device__ __forceinline__ unsigned ploc_block_keep(bool keep, unsigned* wsum) {
-    const unsigned bal = __ballot_sync(0xFFFFFFFFu, keep);
-    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = __popc(bal);
-    __syncthreads();
-    return bal;
-}
-
-// merge of mutual nearest neighbours: a binary node (left, right) with its parent links, in the
-// left cluster's place; per block the number of clusters kept
-__global__ void __launch_bounds__(kPlocThreads) k_ploc_merge(int n, const unsigned* __restrict__ count_p,
-                                                             const int* __restrict__ nn, int* __restrict__ cid,
-                                                             float4* __restrict__ cb, float4* __restrict__ nodes,
-                                                             int* __restrict__ parent, unsigned* __restrict__ next_node,
-                                                             unsigned* __restrict__ blk) {
-    __shared__ unsigned wsum[kPlocThreads / 32];
-    const int count = (int)*count_p;
-    const int b0 = blockIdx.x * kPlocThreads;
-    if (b0 >= count) return;
-    const int i = b0 + threadIdx.x;
-    bool keep = false;
-    if (i < count) {
-        const int j = nn[i];
-        const bool mutual = j >= 0 && nn[j] == i;
-        keep = !(mutual && j < i);
-        if (mutual && i < j) {
-            const int idx = (int)atomicSub(next_node, 1u) - 1;
-            const int l = cid[i], r = cid[j];
-            nodes[4 * (size_t)idx + 3] = make_float4(__int_as_float(l), __int_as_float(r), 0.0f, 0.0f);
-            parent[l < 0 ? (n - 1) + ~l : l] = idx;
-            parent[r < 0 ? (n - 1) + ~r : r] = idx;
-            const float4 alo = cb[2 * (size_t)i], ahi = cb[2 * (size_t)i + 1];
-            const float4 blo = cb[2 * (size_t)j], bhi = cb[2 * (size_t)j + 1];
-            cb[2 * (size_t)i] = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
-            cb[2 * (size_t)i + 1] = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
-            cid[i] = idx;
-        }
-    }
-    ploc_block_keep(keep, wsum);
-    if (threadIdx.x == 0) {
-        unsigned s = 0;
-        for (int w = 0; w < kPlocThreads / 32; ++w) s += wsum[w];
-        blk[blockIdx.x] = s;
-    }
-}
-
-// exclusive scan of the per-block counts in one block; the total is the next cluster count
-__global__ void __launch_bounds__(kPlocScanThreads) k_ploc_scan(const unsigned* __restrict__ count_p,
-                                                                unsigned* __restrict__ blk,
-                                                                unsigned* __restrict__ count_out) {
-    __shared__ unsigned wsum[kPlocScanThreads / 32];
-    const int count = (int)*count_p;
-    const int nb = (count + kPlocThreads - 1) / kPlocThreads;
-    const unsigned ln = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    unsigned carry = 0;
-    for (int base = 0; base < nb; base += kPlocScanThreads) {
-        const int k = base + (int)threadIdx.x;
-        const unsigned v = k < nb ? blk[k] : 0u;
-        unsigned x = v;  // inclusive scan within the warp
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-            if (ln >= (unsigned)o) x += y;
-        }
-        if (ln == 31) wsum[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            unsigned t = wsum[ln];
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned y = __shfl_up_sync(0xFFFFFFFFu, t, o);
-                if (ln >= (unsigned)o) t += y;
+    const int i = b0 - kPlocRadius + (int)threadIdx.x;
+    int best = -1;
+    if (i >= 0 && i < count) {
+        const int s = threadIdx.x + kPlocRadius;
+        const float4 lo = slo[s], hi = shi[s];
+        float barea = INFINITY;
+        // nearer positions first, so a farther one has to be strictly smaller. At one distance the pairs (i - d, i)
+        // and (i, i + d) are ordered by the parity of the lower index, then by the index: coincident Gaussians
+        // pair up as (0,1), (2,3), ... and halve every iteration, where the smaller index alone would merge one pair
+        // an iteration
+#pragma unroll 4
+        for (int d = 1; d <= kPlocRadius; ++d) {
+            const bool has_l = i - d >= 0, has_r = i + d < count;
+            const float al = has_l ? ploc_area(lo, hi, slo[s - d], shi[s - d]) : 0.0f;
+            const float ar = has_r ? ploc_area(lo, hi, slo[s + d], shi[s + d]) : 0.0f;
+            const bool tie_left = (d & 1) == 0 || (i & 1) != 0;
+            const bool left = has_l && (!has_r || al < ar || (al == ar && tie_left));
+            const float a = left ? al : ar;
+            if ((has_l || has_r) && (best < 0 || a < barea)) {
+                barea = a;
+                best = left ? i - d : i + d;
             }
-            wsum[ln] = t;
         }
-        __syncthreads();
-        if (k < nb) blk[k] = carry + (w > 0 ? wsum[w - 1] : 0u) + x - v;
-        carry += wsum[kPlocScanThreads / 32 - 1];
-        __syncthreads();
     }
-    if (threadIdx.x == 0) *count_out = carry;
+    nn[threadIdx.x] = best;
+    __syncthreads();
+    const int k = (int)threadIdx.x - kPlocRadius;  // within the block's own clusters
+    bool keep = false;
+    if (k >= 0 && k < kPlocThreads && i < count) {
+        const int j = best;
+        const bool mutual = j >= 0 && nn[j - (b0 - kPlocRadius)] == i;
+        partner[i] = mutual ? j : -1;
+        keep = !(mutual && j < i);
+    }
+    const unsigned bal = __ballot_sync(0xFFFFFFFFu, keep);
+    if ((threadIdx.x & 31) == 0 && bal) atomicAdd(&kept, __popc(bal));
+    __syncthreads();
+    if (threadIdx.x == 0) blk[blockIdx.x] = kept;
 }
 
-// the kept clusters, in order, into the other list
-__global__ void __launch_bounds__(kPlocThreads) k_ploc_compact(const unsigned* __restrict__ count_p,
-                                                               const int* __restrict__ nn, const int* __restrict__ cid,
-                                                               const float4* __restrict__ cb,
-                                                               const unsigned* __restrict__ blk, int* __restrict__ cid_out,
-                                                               float4* __restrict__ cb_out) {
-    __shared__ unsigned wsum[kPlocThreads / 32];
+__global__ void __launch_bounds__(kPlocThreads) k_ploc_merge(int n, const unsigned* __restrict__ count_p,
+                                                             const int* __restrict__ partner, const int* __restrict__ cid,
+                                                             const float4* __restrict__ cb,
+                                                             const unsigned* __restrict__ blk, int* __restrict__ cid_out,
+                                                             float4* __restrict__ cb_out, float4* __restrict__ nodes,
+                                                             int* __restrict__ parent, unsigned* __restrict__ next_node,
+                                                             unsigned* __restrict__ count_out) {
+    __shared__ unsigned wsum[kPlocThreads / 32], wbefore[kPlocThreads / 32];
     const int count = (int)*count_p;
     const int b0 = blockIdx.x * kPlocThreads;
     if (b0 >= count) return;
+    unsigned before = 0;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += kPlocThreads) before += blk[k];
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
     const int i = b0 + threadIdx.x;
-    bool keep = false;
-    if (i < count) {
-        const int j = nn[i];
-        keep = !(j >= 0 && j < i && nn[j] == i);
+    const int j = i < count ? partner[i] : -1;
+    const bool keep = i < count && !(j >= 0 && j < i);
+    const unsigned bal = __ballot_sync(0xFFFFFFFFu, keep);
+    if ((threadIdx.x & 31) == 0) {
+        wsum[threadIdx.x >> 5] = __popc(bal);
+        wbefore[threadIdx.x >> 5] = before;
     }
-    const unsigned bal = ploc_block_keep(keep, wsum);
-    unsigned off = blk[blockIdx.x] + __popc(bal & ((1u << (threadIdx.x & 31u)) - 1u));
-    for (unsigned w = 0; w < (threadIdx.x >> 5); ++w) off += wsum[w];
-    if (keep) {
-        cid_out[off] = cid[i];
-        cb_out[2 * (size_t)off] = cb[2 * (size_t)i];
-        cb_out[2 * (size_t)off + 1] = cb[2 * (size_t)i + 1];
+    __syncthreads();
+    unsigned off = __popc(bal & ((1u << (threadIdx.x & 31u)) - 1u)), own = 0;
+    for (unsigned w = 0; w < kPlocThreads / 32; ++w) {
+        off += wbefore[w] + (w < (threadIdx.x >> 5) ? wsum[w] : 0u);
+        own += wbefore[w] + wsum[w];
     }
+    if (threadIdx.x == 0 && b0 + kPlocThreads >= count) *count_out = own;
+    if (!keep) return;
+    int id = cid[i];
+    float4 lo = cb[2 * (size_t)i], hi = cb[2 * (size_t)i + 1];
+    if (j >= 0) {
+        const int idx = (int)atomicSub(next_node, 1u) - 1;
+        const int r = cid[j];
+        nodes[4 * (size_t)idx + 3] = make_float4(__int_as_float(id), __int_as_float(r), 0.0f, 0.0f);
+        parent[id < 0 ? (n - 1) + ~id : id] = idx;
+        parent[r < 0 ? (n - 1) + ~r : r] = idx;
+        const float4 blo = cb[2 * (size_t)j], bhi = cb[2 * (size_t)j + 1];
+        lo = make_float4(fminf(lo.x, blo.x), fminf(lo.y, blo.y), fminf(lo.z, blo.z), 0.0f);
+        hi = make_float4(fmaxf(hi.x, bhi.x), fmaxf(hi.y, bhi.y), fmaxf(hi.z, bhi.z), 0.0f);
+        id = idx;
+    }
+    cid_out[off] = id;
+    cb_out[2 * (size_t)off] = lo;
+    cb_out[2 * (size_t)off + 1] = hi;
 }
 
 // A pair's place in the order of the pairs (area, list distance, parity of the lower index, lower index) as the
-// neighbour search of k_ploc_nn ranks them.
+// neighbour search of k_ploc_pair ranks them.
 struct PlocPair {
     float area;
     int dist, lower, other;  // other: the neighbour, -1 none
@@ -429,10 +396,10 @@ __device__ __forceinline__ bool ploc_before(const PlocPair& a, const PlocPair& b
 
 // The iterations from kPlocTail clusters to the root, in one block with the list in shared memory. Most of a build's
 // iterations are here: the last few thousand clusters merge a few pairs at a time (a million Gaussians take about
-// 16 iterations to 3000 clusters and 110 from there), and as launches each cost four kernels of a few us and a
+// 70 iterations to 3000 clusters and 60 from there), and as launches each cost four kernels of a few us and a
 // quarter of a host round trip. As many lanes as fit share the search of a cluster's 32 neighbours; the
-// order of pairs is strict, so the pairs are those of k_ploc_nn and k_ploc_merge. Bound by the latency of the
-// iteration (search, merge, scan): a rebuild of a million Gaussians took 10.75 ms and takes TIMED with this kernel,
+// order of pairs is strict, so the pairs are those of k_ploc_pair. Bound by the latency of the
+// iteration (search, merge, scan): a rebuild of a million Gaussians took 10.75 ms and takes 4.3 with this kernel,
 // the collapse in parallel (k_collapse_level) and the scratch kept.
 struct PlocTail {
     float box[2][6][kPlocTail];
@@ -852,17 +819,15 @@ cudaError_t ploc_build(AccelState& st, int n, cudaStream_t s, std::string& err) 
     e = cudaGetLastError();
     int cur = 0;
     long long left = n;
-    // an iteration merges about a third of the clusters: the first read comes when the list might be short
+    // an iteration merges some 8 % of the clusters: the first read comes when the list might be short
     int batch = 0;
-    for (double c = n; c > kPlocTail; c *= 0.66) ++batch;
+    for (double c = n; c > kPlocTail; c *= 0.9) ++batch;
     for (long long it = 0; e == cudaSuccess && left > kPlocTail; batch = kPlocBatch) {
         const unsigned blocks = (unsigned)((left + kPlocThreads - 1) / kPlocThreads);
         for (int b = 0; b < batch; ++b, ++it) {
-            k_ploc_nn<<<blocks, kPlocThreads, 0, s>>>(cnt + cur, cb[cur], nn);
-            k_ploc_merge<<<blocks, kPlocThreads, 0, s>>>(n, cnt + cur, nn, cid[cur], cb[cur], st.nodes, st.parent,
-                                                         next_node, blk);
-            k_ploc_scan<<<1, kPlocScanThreads, 0, s>>>(cnt + cur, blk, cnt + 1 - cur);
-            k_ploc_compact<<<blocks, kPlocThreads, 0, s>>>(cnt + cur, nn, cid[cur], cb[cur], blk, cid[1 - cur], cb[1 - cur]);
+            k_ploc_pair<<<blocks, kPlocPairThreads, 0, s>>>(cnt + cur, cb[cur], nn, blk);
+            k_ploc_merge<<<blocks, kPlocThreads, 0, s>>>(n, cnt + cur, nn, cid[cur], cb[cur], blk, cid[1 - cur], cb[1 - cur],
+                                                         st.nodes, st.parent, next_node, cnt + 1 - cur);
             cur = 1 - cur;
         }
         e = cudaGetLastError();
