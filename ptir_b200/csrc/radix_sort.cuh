@@ -1,13 +1,14 @@
 // Stable LSD radix sort of (key, value) pairs on the device: the sort of the LBVH build (60-bit
 // Morton keys) and of the wavefront's ray order (28-bit keys).
 //
-// Each pass sorts by one 8-bit digit. The items are split into warp tiles of kRsItemsPerWarp
-// consecutive items. A pass is three steps:
+// Each pass sorts by one 8-bit digit. The items are split into warp tiles of consecutive items, 2048 or 512 of
+// them (rs_items). The number of items may be known on the device only (`count`, at most the host's n): tiles past
+// it are empty. A pass is three steps:
 //   1. count: every warp counts its tile's digits in a shared-memory histogram and writes the
 //      256 counts, digit-major (counts[digit * tiles + tile]);
 //   2. scan: an exclusive prefix sum over those counts, so that counts[digit * tiles + tile]
-//      becomes where the tile's first item of that digit goes (reduce, scan of the block sums,
-//      apply);
+//      becomes where the tile's first item of that digit goes (by one block up to kRsScanOne counts, else
+//      reduce, scan of the block sums, apply);
 //   3. scatter: every warp walks its tile again in order, 32 items at a time. Lanes with the same
 //      digit find each other with __match_any_sync; an item's place is its digit's running
 //      offset plus the number of same-digit lanes before it, and the highest of them advances
@@ -25,12 +26,16 @@ namespace ptir {
 constexpr int kRsBits = 8;
 constexpr int kRsBuckets = 1 << kRsBits;
 constexpr int kRsWarps = 8;                // warps per block of the count and scatter kernels
-constexpr int kRsItemsPerWarp = 2048;      // consecutive items of a warp tile
+constexpr int kRsScanOne = 1 << 16;        // counts up to which one block scans them
 constexpr int kRsScanThreads = 1024;
 constexpr int kRsScanItems = 4;            // per thread of a scan block
 constexpr int kRsScanTile = kRsScanThreads * kRsScanItems;
 
-inline long long rs_tiles(long long n) { return (n + kRsItemsPerWarp - 1) / kRsItemsPerWarp; }
+// Items of a warp tile. A warp walks its tile 32 items at a time, each step waiting for the one before, so a sort of
+// less than 4M items with 2048 a warp leaves SMs without work: a million 64-bit keys took 55 us a scatter pass
+// with 2048 items (61 blocks) and 23 us with 512.
+inline int rs_items(long long n) { return n < (1ll << 22) ? 512 : 2048; }
+inline long long rs_tiles(long long n) { return (n + rs_items(n) - 1) / rs_items(n); }
 inline long long rs_scan_blocks(long long m) { return (m + kRsScanTile - 1) / kRsScanTile; }
 
 template <class Key>
@@ -38,18 +43,26 @@ __device__ __forceinline__ unsigned rs_digit(Key k, int shift, unsigned mask) {
     return (unsigned)(k >> shift) & mask;
 }
 
+// the items: the device's count when there is one
+__device__ __forceinline__ long long rs_count(long long n, const unsigned* count) {
+    return count ? ((long long)*count < n ? (long long)*count : n) : n;
+}
+
 template <class Key>
-__global__ void __launch_bounds__(kRsWarps * 32) k_rs_count(const Key* __restrict__ keys, long long n, int shift,
-                                                            unsigned mask, unsigned* __restrict__ counts,
+__global__ void __launch_bounds__(kRsWarps * 32) k_rs_count(const Key* __restrict__ keys, long long n_max,
+                                                            const unsigned* __restrict__ count, unsigned above, int items,
+                                                            int shift, unsigned mask, unsigned* __restrict__ counts,
                                                             long long tiles) {
+    const long long n = rs_count(n_max, count);
+    if (n <= (long long)above) return;
     __shared__ unsigned hist[kRsWarps][kRsBuckets];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long tile = (long long)blockIdx.x * kRsWarps + w;
     for (int d = lane; d < kRsBuckets; d += 32) hist[w][d] = 0u;
     __syncwarp();
     if (tile < tiles) {
-        const long long begin = tile * kRsItemsPerWarp;
-        const long long end = begin + kRsItemsPerWarp < n ? begin + kRsItemsPerWarp : n;
+        const long long begin = tile * items;
+        const long long end = begin + items < n ? begin + items : n;
         for (long long i = begin + lane; i < end; i += 32) atomicAdd(&hist[w][rs_digit(keys[i], shift, mask)], 1u);
         __syncwarp();
         for (int d = lane; d < kRsBuckets; d += 32) counts[(long long)d * tiles + tile] = hist[w][d];
@@ -60,7 +73,9 @@ __global__ void __launch_bounds__(kRsWarps * 32) k_rs_count(const Key* __restric
 
 // block sums of the scan tiles
 static __global__ void __launch_bounds__(kRsScanThreads) k_rs_scan_reduce(const unsigned* __restrict__ v, long long m,
-                                                                   unsigned* __restrict__ partial) {
+                                                                   unsigned* __restrict__ partial,
+                                                                   const unsigned* __restrict__ count, unsigned above) {
+    if (count && *count <= above) return;
     __shared__ unsigned warp_sums[kRsScanThreads / 32];
     const long long base = (long long)blockIdx.x * kRsScanTile;
     unsigned s = 0;
@@ -104,7 +119,9 @@ static __device__ __forceinline__ unsigned rs_block_exclusive(unsigned x, unsign
 }
 
 // exclusive scan of the block sums, in place, by one block walking them in chunks
-static __global__ void __launch_bounds__(kRsScanThreads) k_rs_scan_partials(unsigned* __restrict__ partial, long long nb) {
+static __global__ void __launch_bounds__(kRsScanThreads) k_rs_scan_partials(unsigned* __restrict__ partial, long long nb,
+                                                                     const unsigned* __restrict__ count, unsigned above) {
+    if (count && *count <= above) return;
     __shared__ unsigned warp_sums[kRsScanThreads / 32];
     unsigned carry = 0;
     for (long long base = 0; base < nb; base += kRsScanThreads) {
@@ -119,7 +136,9 @@ static __global__ void __launch_bounds__(kRsScanThreads) k_rs_scan_partials(unsi
 
 // exclusive scan of each tile, offset by its block's scanned sum
 static __global__ void __launch_bounds__(kRsScanThreads) k_rs_scan_apply(unsigned* __restrict__ v, long long m,
-                                                                  const unsigned* __restrict__ partial) {
+                                                                  const unsigned* __restrict__ partial,
+                                                                  const unsigned* __restrict__ count, unsigned above) {
+    if (count && *count <= above) return;
     __shared__ unsigned warp_sums[kRsScanThreads / 32];
     const long long base = (long long)blockIdx.x * kRsScanTile;
     // each thread owns kRsScanItems consecutive values
@@ -138,21 +157,40 @@ static __global__ void __launch_bounds__(kRsScanThreads) k_rs_scan_apply(unsigne
     }
 }
 
+// exclusive scan of up to kRsScanOne values, in place, by one block
+static __global__ void __launch_bounds__(kRsScanThreads) k_rs_scan_one(unsigned* __restrict__ v, int m,
+                                                                       const unsigned* __restrict__ count, unsigned above) {
+    __shared__ unsigned warp_sums[kRsScanThreads / 32];
+    if (count && *count <= above) return;
+    unsigned carry = 0;
+    for (int base = 0; base < m; base += kRsScanTile) {
+        const int first = base + (int)threadIdx.x * kRsScanItems;
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (first < m) x = *reinterpret_cast<const uint4*>(v + first);  // m is a multiple of the 256 buckets
+        unsigned total;
+        const unsigned run = carry + rs_block_exclusive(x.x + x.y + x.z + x.w, warp_sums, total);
+        if (first < m) *reinterpret_cast<uint4*>(v + first) = make_uint4(run, run + x.x, run + x.x + x.y, run + x.x + x.y + x.z);
+        carry += total;
+    }
+}
+
 template <class Key>
 __global__ void __launch_bounds__(kRsWarps * 32) k_rs_scatter(const Key* __restrict__ keys_in,
                                                               const unsigned* __restrict__ vals_in,
                                                               Key* __restrict__ keys_out, unsigned* __restrict__ vals_out,
-                                                              long long n, int shift, unsigned mask,
+                                                              long long n_max, const unsigned* __restrict__ count,
+                                                              unsigned above, int items, int shift, unsigned mask,
                                                               const unsigned* __restrict__ offsets, long long tiles) {
     __shared__ unsigned run[kRsWarps][kRsBuckets];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long tile = (long long)blockIdx.x * kRsWarps + w;
-    if (tile >= tiles) return;  // whole warps leave together
+    const long long n = rs_count(n_max, count);
+    if (tile >= tiles || n <= (long long)above || tile * items >= n) return;  // whole warps leave together
     for (int d = lane; d < kRsBuckets; d += 32) run[w][d] = offsets[(long long)d * tiles + tile];
     __syncwarp();
     const unsigned below = (1u << lane) - 1u;
-    const long long begin = tile * kRsItemsPerWarp;
-    for (int c = 0; c < kRsItemsPerWarp; c += 32) {
+    const long long begin = tile * items;
+    for (int c = 0; c < items; c += 32) {
         const long long i = begin + c + lane;
         const bool valid = i < n;
         Key k = Key(0);
@@ -177,25 +215,33 @@ __global__ void __launch_bounds__(kRsWarps * 32) k_rs_scatter(const Key* __restr
     }
 }
 
-// scratch bytes of radix_sort_pairs for n items with keys of type Key
+// counts of the tiles of n items, at most: not less for a smaller n, whose tiles may be smaller
+inline long long rs_most_counts(long long n) {
+    const long long small = rs_tiles(n < (1ll << 22) ? n : (1ll << 22) - 1), large = (n + 2047) / 2048;
+    return (long long)kRsBuckets * (small > large ? small : large);
+}
+
+// scratch bytes of radix_sort_pairs for n items with keys of type Key (enough for fewer items too)
 template <class Key>
 size_t radix_sort_temp_bytes(long long n) {
-    const long long tiles = rs_tiles(n), m = (long long)kRsBuckets * tiles;
+    const long long m = rs_most_counts(n);
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     return up(sizeof(Key) * (size_t)n) + up(sizeof(unsigned) * (size_t)n) + up(sizeof(unsigned) * (size_t)m) +
            up(sizeof(unsigned) * (size_t)rs_scan_blocks(m));
 }
 
 // Stable sort of (keys_in, vals_in) by bits [begin_bit, end_bit) of the keys into (keys_out,
-// vals_out); `temp` holds radix_sort_temp_bytes<Key>(n) bytes.
+// vals_out); `temp` holds radix_sort_temp_bytes<Key>(n) bytes. With `count` (device) only its first *count items are
+// sorted, and nothing is done when they are `above` or fewer.
 template <class Key>
 cudaError_t radix_sort_pairs(void* temp, size_t temp_bytes, const Key* keys_in, Key* keys_out,
                              const unsigned* vals_in, unsigned* vals_out, long long n, int begin_bit, int end_bit,
-                             cudaStream_t s) {
+                             cudaStream_t s, const unsigned* count = nullptr, unsigned above = 0u) {
     if (n <= 0) return cudaSuccess;
     if (temp_bytes < radix_sort_temp_bytes<Key>(n) || end_bit <= begin_bit || end_bit > (int)(8 * sizeof(Key)))
         return cudaErrorInvalidValue;
     const long long tiles = rs_tiles(n), m = (long long)kRsBuckets * tiles, nb = rs_scan_blocks(m);
+    const int items = rs_items(n);
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     char* p = static_cast<char*>(temp);
     Key* alt_keys = reinterpret_cast<Key*>(p);
@@ -217,11 +263,16 @@ cudaError_t radix_sort_pairs(void* temp, size_t temp_bytes, const Key* keys_in, 
         const bool to_out = ((passes - 1 - pass) & 1) == 0;
         Key* dst_k = to_out ? keys_out : alt_keys;
         unsigned* dst_v = to_out ? vals_out : alt_vals;
-        k_rs_count<Key><<<grid, kRsWarps * 32, 0, s>>>(src_k, n, shift, mask, counts, tiles);
-        k_rs_scan_reduce<<<(unsigned)nb, kRsScanThreads, 0, s>>>(counts, m, partial);
-        k_rs_scan_partials<<<1, kRsScanThreads, 0, s>>>(partial, nb);
-        k_rs_scan_apply<<<(unsigned)nb, kRsScanThreads, 0, s>>>(counts, m, partial);
-        k_rs_scatter<Key><<<grid, kRsWarps * 32, 0, s>>>(src_k, src_v, dst_k, dst_v, n, shift, mask, counts, tiles);
+        k_rs_count<Key><<<grid, kRsWarps * 32, 0, s>>>(src_k, n, count, above, items, shift, mask, counts, tiles);
+        if (m <= kRsScanOne) {
+            k_rs_scan_one<<<1, kRsScanThreads, 0, s>>>(counts, (int)m, count, above);
+        } else {
+            k_rs_scan_reduce<<<(unsigned)nb, kRsScanThreads, 0, s>>>(counts, m, partial, count, above);
+            k_rs_scan_partials<<<1, kRsScanThreads, 0, s>>>(partial, nb, count, above);
+            k_rs_scan_apply<<<(unsigned)nb, kRsScanThreads, 0, s>>>(counts, m, partial, count, above);
+        }
+        k_rs_scatter<Key><<<grid, kRsWarps * 32, 0, s>>>(src_k, src_v, dst_k, dst_v, n, count, above, items, shift, mask,
+                                                         counts, tiles);
         src_k = dst_k;
         src_v = dst_v;
     }

@@ -117,10 +117,8 @@ PTIR_DEV void write_pbr(const FwdOutputs& O, size_t li, const PathState& ps) {
 // per axis of the scene bounds), then the Morton code of its direction's cell within the octant
 // (4 bits per axis of the normalised |d|): 27 bits. Coarse origin cells with fine direction cells keep
 // the rays of a warp on similar traversals; against octant + 8-bit origin cells alone this cut
-// the intersection stage by 7 % on the 1M-Gaussian scene. Queue entries past the count get
-// kSortPad, above all.
-constexpr int kSortKeyBits = 28;
-constexpr unsigned kSortPad = 1u << 27;
+// the intersection stage by 7 % on the 1M-Gaussian scene.
+constexpr int kSortKeyBits = 27;
 
 PTIR_DEV unsigned spread3_8(unsigned v) {
     v &= 0xFFu;
@@ -132,8 +130,10 @@ PTIR_DEV unsigned spread3_8(unsigned v) {
 
 // Keys of queue in_q: the intersect queue's segment rays, or the shadow queue's rays toward their
 // light samples.
-__global__ void __launch_bounds__(kMaxThreads) k_wf_sort_keys(TraceParams P, WfView W, int in_q, unsigned* keys) {
+__global__ void __launch_bounds__(kMaxThreads) k_wf_sort_keys(TraceParams P, WfView W, int in_q, unsigned* keys,
+                                                              unsigned quad_rays) {
     const unsigned count = W.count[in_q];
+    if (count <= quad_rays) return;
     float3 lo = f3(0.0f), scale = f3(0.0f);
     if (P.accel.n > 0) {
         const float4 a = __ldg(P.accel.bounds), b = __ldg(P.accel.bounds + 1);
@@ -141,29 +141,25 @@ __global__ void __launch_bounds__(kMaxThreads) k_wf_sort_keys(TraceParams P, WfV
         scale = make_float3(255.0f / fmaxf(b.x - a.x, 1e-30f), 255.0f / fmaxf(b.y - a.y, 1e-30f),
                             255.0f / fmaxf(b.z - a.z, 1e-30f));
     }
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < W.slots; i += gridDim.x * blockDim.x) {
-        unsigned key = kSortPad;
-        if (i < count) {
-            const unsigned q = W.q[in_q][i];
-            float3 o = W.seg[q].o, d = W.seg[q].d;
-            if (in_q == kQShadow) {
-                d = W.ps[q].em.dir;
-                o = W.seg[q].pos + d * 2e-2f;
-            }
-            const unsigned oct = (d.x < 0.0f ? 4u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 1u : 0u);
-            const float3 c = (o - lo) * scale * (1.0f / 16.0f);
-            const unsigned cx = (unsigned)fminf(fmaxf(c.x, 0.0f), 15.0f);
-            const unsigned cy = (unsigned)fminf(fmaxf(c.y, 0.0f), 15.0f);
-            const unsigned cz = (unsigned)fminf(fmaxf(c.z, 0.0f), 15.0f);
-            const float dn = rsqrtf(fmaxf(dot(d, d), 1e-30f));
-            const unsigned dx = (unsigned)fminf(fabsf(d.x) * dn * 16.0f, 15.0f);
-            const unsigned dy = (unsigned)fminf(fabsf(d.y) * dn * 16.0f, 15.0f);
-            const unsigned dz = (unsigned)fminf(fabsf(d.z) * dn * 16.0f, 15.0f);
-            const unsigned ocell = (spread3_8(cx) << 2) | (spread3_8(cy) << 1) | spread3_8(cz);
-            const unsigned dcell = (spread3_8(dx) << 2) | (spread3_8(dy) << 1) | spread3_8(dz);
-            key = (oct << 24) | (ocell << 12) | dcell;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const unsigned q = W.q[in_q][i];
+        float3 o = W.seg[q].o, d = W.seg[q].d;
+        if (in_q == kQShadow) {
+            d = W.ps[q].em.dir;
+            o = W.seg[q].pos + d * 2e-2f;
         }
-        keys[i] = key;
+        const unsigned oct = (d.x < 0.0f ? 4u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 1u : 0u);
+        const float3 c = (o - lo) * scale * (1.0f / 16.0f);
+        const unsigned cx = (unsigned)fminf(fmaxf(c.x, 0.0f), 15.0f);
+        const unsigned cy = (unsigned)fminf(fmaxf(c.y, 0.0f), 15.0f);
+        const unsigned cz = (unsigned)fminf(fmaxf(c.z, 0.0f), 15.0f);
+        const float dn = rsqrtf(fmaxf(dot(d, d), 1e-30f));
+        const unsigned dx = (unsigned)fminf(fabsf(d.x) * dn * 16.0f, 15.0f);
+        const unsigned dy = (unsigned)fminf(fabsf(d.y) * dn * 16.0f, 15.0f);
+        const unsigned dz = (unsigned)fminf(fabsf(d.z) * dn * 16.0f, 15.0f);
+        const unsigned ocell = (spread3_8(cx) << 2) | (spread3_8(cy) << 1) | spread3_8(cz);
+        const unsigned dcell = (spread3_8(dx) << 2) | (spread3_8(dy) << 1) | spread3_8(dz);
+        keys[i] = (oct << 24) | (ocell << 12) | dcell;
     }
 }
 
@@ -1076,7 +1072,7 @@ static void launch_shadow(int ks, const TraceParams& q, const WfView& W, int B, 
         if (W.slots > quad_rays) fn<<<blocks(grid_cached((const void*)fn, B, 0), B), B, 0, s>>>(q, W, R, items, quad_rays);
     };
     const auto quads = [&](auto* fn) {
-        fn<<<blocks(grid_cached((const void*)fn, B, stacks), B / 32), B, stacks, s>>>(q, W, (R + 3) / 4, items, kQuadRays);
+        fn<<<blocks(grid_cached((const void*)fn, B, stacks), B / 32), B, stacks, s>>>(q, W, (R + 3) / 4, W.q[kQShadow], kQuadRays);
     };
     switch (ks) {
     case 8: quads(k_wf_shadow_quad<8>); lanes(k_wf_shadow<8>, kQuadRays); break;
@@ -1208,19 +1204,25 @@ static WfView view_of(const WavefrontBuffers& b, unsigned long long tile0, unsig
 
 static unsigned long long total_tiles(const TraceParams& p) { return (unsigned long long)p.tiles; }
 
-// The intersect queue in ray order (or as queued when sorting is off): keys, then a key/slot
-// radix sort of the whole chunk capacity (the count stays on the device).
+// Queue in_q in ray order (or as queued when sorting is off): keys, then a key/slot radix sort of what the queue
+// holds (the count stays on the device).
 static const unsigned* sort_queue(const TraceParams& p, const WavefrontBuffers& b, const WfView& W,
-                                  const WavefrontTuning& tune, const StageCtx& sc, cudaStream_t s, int in_q = kQIsect) {
+                                  const WavefrontTuning& tune, const StageCtx& sc, cudaStream_t s, bool quads,
+                                  int in_q = kQIsect) {
     if (!tune.sort_rays) return W.q[in_q];
+    // up to kQuadRays rays are traced by quads, in queue order: each waits for its own ray, and sorting cost more than
+    // it gave (16k rays over 10k Gaussians: a trace of 1.29 ms against 1.69, the stage's time the same; 90k
+    // over 300k: 36.0 against 36.6). How many rays the queue holds only the device knows.
+    const unsigned quad_rays = quads ? kQuadRays : 0u;
+    if (W.slots <= quad_rays) return W.q[in_q];
     unsigned* keys_in = static_cast<unsigned*>(b.sort_keys[0]);
     unsigned* keys_out = static_cast<unsigned*>(b.sort_keys[1]);
     unsigned* sorted = static_cast<unsigned*>(b.sorted);
     const int grid = grid_cached((const void*)k_wf_sort_keys, tune.block);
     sc.run(kStageSort, p, s, [&](const TraceParams& q) {
-        k_wf_sort_keys<<<grid, tune.block, 0, s>>>(q, W, in_q, keys_in);
+        k_wf_sort_keys<<<grid, tune.block, 0, s>>>(q, W, in_q, keys_in, quad_rays);
         radix_sort_pairs<unsigned>(b.sort_temp, b.sort_temp_bytes, keys_in, keys_out, W.q[in_q], sorted,
-                                   (long long)W.slots, 0, kSortKeyBits, s);
+                                   (long long)W.slots, 0, kSortKeyBits, s, W.count + in_q, quad_rays);
     });
     return sorted;
 }
@@ -1283,8 +1285,11 @@ static void run_trace(const TraceLaunch& l, long long rays, const TraceParams& q
     int refill;
     void* args[] = {&p, &vis, &w, &in_q, &items, &out_q, &cursor, &refill, &quad_rays};
     if (l.quad_fn) {
+        const unsigned* sorted = items;
+        items = W.q[in_q];  // as queued (sort_queue)
         refill = l.quad_refill;
         cudaLaunchKernel(l.quad_fn, blocks(l.quad_grid, l.block / 32), dim3((unsigned)l.block), args, quad_smem(l.block), s);
+        items = sorted;
     }
     if (rays > (long long)quad_rays) {
         refill = l.lane_refill;
@@ -1325,7 +1330,7 @@ static cudaError_t run_fwd(const TraceParams& p, const FwdOutputs& o, WavefrontB
             k_wf_fwd_primary<K><<<std::min(g_primary, cap), B, 0, s>>>(q, o, W);
         });
         if (p.flags & kMis) {
-            const unsigned* shadow_items = sort_queue(p, b, W, tune, sc, s, kQShadow);
+            const unsigned* shadow_items = sort_queue(p, b, W, tune, sc, s, tune.shadow_kbuf <= 16, kQShadow);
             sc.run(kStageShadow, p, s,
                    [&](const TraceParams& q) { launch_shadow(tune.shadow_kbuf, q, W, B, R, shadow_items, s); });
         }
@@ -1338,7 +1343,7 @@ static cudaError_t run_fwd(const TraceParams& p, const FwdOutputs& o, WavefrontB
             ++cursor;
             if (depth + 1 >= mb) break;
             cudaMemsetAsync(W.count + kQBounce, 0, sizeof(unsigned), s);
-            const unsigned* items = sort_queue(p, b, W, tune, sc, s);
+            const unsigned* items = sort_queue(p, b, W, tune, sc, s, trace.quad_fn != nullptr);
             sc.run(kStageIntersect, p, s, [&](const TraceParams& q) {
                 run_trace(trace, (long long)nt * 32, q, o.visibility, W, kQIsect, items, kQBounce, cursor, s);
             });
@@ -1386,7 +1391,7 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
             k_wb_primary<K><<<std::min(g_primary, cap), B, 0, s>>>(q, bi, W);
         });
         if (p.flags & kMis) {
-            const unsigned* shadow_items = sort_queue(p, b, W, tune, sc, s, kQShadow);
+            const unsigned* shadow_items = sort_queue(p, b, W, tune, sc, s, tune.shadow_kbuf <= 16, kQShadow);
             sc.run(kStageShadow, p, s,
                    [&](const TraceParams& q) { launch_shadow(tune.shadow_kbuf, q, W, B, R, shadow_items, s); });
         }
@@ -1404,7 +1409,7 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
             ++cursor;
             if (depth + 1 >= mb) break;
             cudaMemsetAsync(W.count + kQBounce, 0, sizeof(unsigned), s);
-            const unsigned* items = sort_queue(p, b, W, tune, sc, s);
+            const unsigned* items = sort_queue(p, b, W, tune, sc, s, trace.quad_fn != nullptr);
             sc.run(kStageIntersect, p, s, [&](const TraceParams& q) {
                 run_trace(trace, (long long)nt * 32, q, nullptr, W, kQIsect, items, kQBounce, cursor, s);
             });
