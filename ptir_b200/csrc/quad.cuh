@@ -206,4 +206,209 @@ PTIR_DEV bool quad_step(const AccelView& A, float3 o, float3 d, QuadTrace<K>& t,
     return more;
 }
 
+// ------------------------------------------------------------------------------------
+// Resumed calls (traverse.cuh) of a quad: what a call sets aside is appended to the quad's frontier, the entries of
+// one step together, in the order in which the one-lane call sets them aside; so the next call comes to
+// the same entries in the same order.
+
+// A quad's frontier: two buffers of `cap` (code, lower bound) entries, as Frontier, and where its calls stand in them.
+struct QuadFrontier {
+    uint2* buf;
+    int cap;
+    int cur, n, pos, next;
+};
+
+constexpr int kQuadPull = (int)0x80000001;  // QuadTrace::node: the call goes on with its frontier
+
+// append the entries of the lanes with `pred`, in lane order
+PTIR_DEV void quad_defer(QuadFrontier& F, bool pred, int code, float lower, unsigned c, unsigned base, unsigned mask) {
+    const unsigned m = (__ballot_sync(mask, pred) >> base) & 15u;
+    if (pred) {
+        const int at = F.next + __popc(m & ((1u << c) - 1u));
+        if (at < F.cap) F.buf[(1 - F.cur) * F.cap + at] = make_uint2((unsigned)code, __float_as_uint(lower));
+    }
+    F.next += __popc(m);
+}
+
+// quad_insert that gives back the entry pushed out of a full buffer (id kNoHit when none), as kbuf_insert_evict:
+// the last entry, or the first of the run of equal distances that ends there
+template <int K>
+PTIR_DEV void quad_insert_evict(QuadTrace<K>& t, float ts, unsigned id, unsigned c, unsigned base, unsigned mask,
+                                float& et, unsigned& eid) {
+    constexpr int L = QuadTrace<K>::L;
+    unsigned run = t.kid[0];
+#pragma unroll
+    for (int j = 1; j < L; ++j) run = t.kt[j] == t.kt[j - 1] ? run : t.kid[j];
+    const float before = __shfl_up_sync(mask, t.kt[L - 1], 1, 4);
+    const unsigned before_run = __shfl_up_sync(mask, run, 1, 4);
+    if (c > 0 && t.kt[L - 1] == t.kt[0] && t.kt[0] == before) run = before_run;
+    et = __shfl_sync(mask, t.kt[L - 1], base + 3u);
+    eid = __shfl_sync(mask, run, base + 3u);
+    if (!(ts < et)) eid = kNoHit;
+    quad_insert(t, ts, id, c, mask);
+}
+
+// trace_start<K, true, true> for a quad: with `resume` the call goes on from what the previous one set aside, unless
+// that overflowed the frontier. The caller synchronises the warp between two calls: the lanes read each other's entries.
+template <int K>
+PTIR_DEV bool quad_start_resume(const AccelView& A, float3 o, float3 d, float tmin, float tend, QuadTrace<K>& t,
+                                QuadFrontier& F, bool resume, TraceCounters& ctr, unsigned c) {
+    if (!resume) F.cur = F.n = F.pos = F.next = 0;
+    if (!quad_start(A, o, d, tmin, tend, t, ctr, c, kFarT)) {
+        if (A.n == 1 && t.kid[0] != kNoHit) t.kid[0] = 0u;  // the k-buffer holds leaf record indices
+        return false;
+    }
+    if (resume && F.next <= F.cap) {
+        F.cur = 1 - F.cur;
+        F.n = F.next;
+        F.pos = F.next = 0;
+        if (F.n == 0) return false;  // nothing was set aside: no candidate remains
+        t.node = kQuadPull;
+    } else {
+        F.n = F.pos = F.next = 0;
+    }
+    return true;
+}
+
+// One step of a resumable call (trace_step<K, true, true>) of the quads in `mask`: a node visit, or up to four
+// consecutive leaves of the frontier. The k-buffer holds leaf record indices. False when the call is complete.
+template <int K>
+PTIR_DEV bool quad_step_resume(const AccelView& A, float3 o, float3 d, QuadTrace<K>& t, QuadFrontier& F, StackEntry* stack,
+                               unsigned* err, TraceCounters& ctr, unsigned ln, unsigned mask) {
+    constexpr int L = QuadTrace<K>::L;
+    const unsigned c = ln & 3u, base = ln & 28u;
+    const bool pulling = t.node == kQuadPull;
+    int child = kNoChild;
+    float t0 = 0.0f, key = 0.0f;
+    bool crossed = false;
+    if (pulling) {
+        const int at = F.pos + (int)c;
+        if (at < F.n) {
+            const uint2 e = F.buf[F.cur * F.cap + at];
+            child = (int)e.x;
+            t0 = __uint_as_float(e.y);
+        }
+    } else {
+        const float3 inv = t.inv;
+        float4 p, q;  // lo.xyz hi.x | hi.yz child kmax
+        ld256(A.quads + 8 * (size_t)t.node + 2 * c, p, q);
+        child = __float_as_int(q.z);
+        const bool px = inv.x >= 0.0f, py = inv.y >= 0.0f, pz = inv.z >= 0.0f;
+        const float3 oi = make_float3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+        const float a = max3f(fmaf(px ? p.x : p.w, inv.x, -oi.x), fmaf(py ? p.y : q.x, inv.y, -oi.y),
+                              fmaxf(fmaf(pz ? p.z : q.y, inv.z, -oi.z), t.tmin));
+        const float b = min3f(fmaf(px ? p.w : p.x, inv.x, -oi.x), fmaf(py ? q.x : p.y, inv.y, -oi.y),
+                              fminf(fmaf(pz ? q.y : p.z, inv.z, -oi.z), t.tend));
+        t0 = a;
+        key = 15.0f * a + b;
+        crossed = child != kNoChild && a <= b;
+        if (c == 0) ++ctr.nodes;
+    }
+    const bool hit = crossed && t0 <= t.tk;
+    quad_defer(F, crossed && !hit, child, t0, c, base, mask);
+    // the leading leaves of a pulled group; a node at its head is visited or set aside by itself
+    const bool pulled = pulling && child != kNoChild && child < 0;
+    const unsigned pm = (__ballot_sync(mask, pulled) >> base) & 15u;
+    const unsigned lead = __ffs(~pm) - 1;  // leaves before the first other entry
+    const bool leaf = pulling ? c < lead : (hit && child < 0);
+    int test = 0;
+    float ts = kFarT;
+    if (leaf) {
+        if (!pulling || t0 <= t.tk) test = leaf_candidate3_wide(A, ~child, o, d, t.tmin, t.tend, t.tk, ts);
+        // (an entry past the K-th distance is set aside below: the K-th distance only falls)
+    }
+    // the leaves in order: set aside, or inserted, what leaves the buffer set aside
+    unsigned mine = (__ballot_sync(mask, leaf) >> base) & 15u;
+    while (__any_sync(mask, mine != 0u)) {
+        const unsigned src = base + (mine ? __ffs(mine) - 1 : 0u);
+        const float ti = __shfl_sync(mask, ts, src), lower = __shfl_sync(mask, t0, src);
+        const int code = __shfl_sync(mask, child, src), tst = __shfl_sync(mask, test, src);
+        const bool live = mine != 0u;
+        const bool past = live && pulling && !(lower <= t.tk);
+        if (live && !past && c == 0) ++ctr.leaves;
+        const bool late = live && !past && tst != 0 && !(ti < t.tk);
+        const bool in = live && !past && !late && tst == 3;
+        float et;
+        unsigned eid;
+        quad_insert_evict(t, in ? ti : kFarT, (unsigned)~code, c, base, mask, et, eid);
+        const bool out = in && eid != kNoHit;
+        quad_defer(F, c == 0 && (past || late || out), out ? ~(int)eid : code, past ? lower : (late ? ti : et), c, base, mask);
+        t.tk = __shfl_sync(mask, t.kt[L - 1], base + 3u);
+        mine &= mine - 1u;
+    }
+    if (pulling) F.pos += (int)lead;
+    // descent
+    const bool child_in = hit && child >= 0;
+    const bool inner = child_in && t0 <= t.tk;
+    quad_defer(F, child_in && !inner, child, t0, c, base, mask);  // passed over after the leaf tests
+    const int ik = inner ? (int)((__float_as_uint(key) & ~3u) | c) : 0x7FFFFFFF;
+    const int k1 = __shfl_xor_sync(mask, ik, 1), k2 = __shfl_xor_sync(mask, ik, 2), k3 = __shfl_xor_sync(mask, ik, 3);
+    const int rank = (k1 < ik ? 1 : 0) + (k2 < ik ? 1 : 0) + (k3 < ik ? 1 : 0);
+    const int best = min(min(ik, k1), min(k2, k3));
+    const int np = __popc((__ballot_sync(mask, inner) >> base) & 15u) - 1;
+    const int next = __shfl_sync(mask, child, base + (best & 3));
+    bool more = true, pop = np < 0;
+    if (!pop) {
+        if (t.sp + np > kStackDepth) {
+            if (c == 0) atomicOr(err, kErrStackOverflow);
+            more = false;
+        } else {
+            if (inner && rank > 0) stack[t.sp + np - rank] = make_int2(child, __float_as_int(t0));
+            t.sp += np;
+            t.node = next;
+        }
+    }
+    __syncwarp(mask);
+    while (__any_sync(mask, pop && t.sp > 0)) {
+        const int i = t.sp - 1 - (int)c;
+        const bool there = pop && i >= 0;
+        StackEntry e = make_int2(0, 0);
+        if (there) e = stack[i];
+        const bool ok = there && __int_as_float(e.y) <= t.tk;
+        const unsigned om = (__ballot_sync(mask, ok) >> base) & 15u;
+        const unsigned first = om ? __ffs(om) - 1 : 4u;
+        quad_defer(F, there && c < first, e.x, __int_as_float(e.y), c, base, mask);
+        const int popped = __shfl_sync(mask, e.x, base + (first & 3u));
+        if (pop && t.sp > 0) {
+            if (om) {
+                t.node = popped;
+                t.sp -= 1 + (int)first;
+                pop = false;
+            } else {
+                t.sp = max(t.sp - 4, 0);
+            }
+        }
+    }
+    // the stack is empty: the next frontier entries. Leaves are left to the next step; a node is visited, or set
+    // aside when it lies past the K-th distance
+    while (__any_sync(mask, pop)) {
+        const int at = F.pos + (int)c;
+        const bool there = pop && at < F.n;
+        uint2 e = make_uint2(0u, 0u);
+        if (there) e = F.buf[F.cur * F.cap + at];
+        const bool is_leaf = there && (int)e.x < 0, visit = there && !is_leaf && __uint_as_float(e.y) <= t.tk;
+        const unsigned sm = (__ballot_sync(mask, is_leaf || visit) >> base) & 15u;
+        const unsigned vm = (__ballot_sync(mask, visit) >> base) & 15u;
+        const unsigned first = sm ? __ffs(sm) - 1 : 4u;
+        quad_defer(F, there && c < first, (int)e.x, __uint_as_float(e.y), c, base, mask);
+        const int code = (int)__shfl_sync(mask, e.x, base + (first & 3u));
+        if (pop) {
+            if (sm) {
+                const bool v = (vm >> first) & 1u;
+                t.node = v ? code : kQuadPull;
+                F.pos += (int)first + (v ? 1 : 0);
+                pop = false;
+            } else {
+                F.pos = min(F.pos + 4, F.n);
+                if (F.pos >= F.n) {
+                    pop = false;
+                    more = false;
+                }
+            }
+        }
+    }
+    if (!more) ctr.candidates += quad_count(t);
+    return more;
+}
+
 }  // namespace ptir

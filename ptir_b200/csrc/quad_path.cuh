@@ -205,4 +205,59 @@ PTIR_DEV bool quad_shadow_walk(const TraceParams& P, const QuadTrace<K>& t, floa
     return occluded;
 }
 
+// replay_batch (path.cuh) for a quad whose k-buffer holds leaf record indices: each lane evaluates its hits and
+// scatters their gradient rows, the transmittance goes through the hits in order.
+template <int K>
+PTIR_DEV void quad_replay_batch(const TraceParams& P, const BwdInputs& B, ReplayState& r, const QuadTrace<K>& t,
+                                TraceCounters& ctr, unsigned ln, unsigned mask) {
+    const unsigned c = ln & 3u, base = ln & 28u;
+    const bool metallic_on = (P.flags & kMetallic) != 0;
+#pragma unroll 1
+    for (int k = 0; k < K / 4; ++k) {
+        float th;
+        unsigned leaf;
+        quad_hit(t, k, c, base, mask, th, leaf);
+        const bool open = r.tr > P.min_transmittance;
+        const bool hit = open && leaf != kNoHit;
+        unsigned id = 0u;
+        float alpha = 0.0f;
+        bool accept = false;
+        if (hit) {
+            id = leaf_gaussian(P.accel, leaf);
+            if (!(r.self_occ && self_occluded(P, th, id, r.d))) {
+                float dns;
+                const Response res = respond(P, id, r.o, r.d, dns);
+                alpha = res.alpha;
+                accept = res.gres > P.min_response && res.alpha > P.alpha_min;
+            }
+        }
+        const unsigned hits = (__ballot_sync(mask, hit) >> base) & 15u;
+        const unsigned acc = (__ballot_sync(mask, accept) >> base) & 15u;
+        float w = 0.0f;
+        bool scatter = false;
+#pragma unroll
+        for (unsigned i = 0; i < 4; ++i) {
+            const float ai = __shfl_sync(mask, alpha, base + i), ti = __shfl_sync(mask, th, base + i);
+            if (!((hits >> i) & 1u) || !(r.tr > P.min_transmittance)) continue;
+            if ((acc >> i) & 1u) {
+                if (i == c) {
+                    w = ai * r.tr;
+                    scatter = true;
+                }
+                r.tr *= (1.0f - ai);
+            }
+            r.start = fmaxf(r.start, ti);
+        }
+        if (scatter) {
+            ++ctr.replay_accepted;
+            float* g = B.particle_material_grad + 5 * (size_t)id;
+            float* cg = B.particle_material_comp ? B.particle_material_comp + 5 * (size_t)id : nullptr;
+            float row[5] = {w * r.da.x, w * r.da.y, w * r.da.z, w * r.dr, w * r.dm};
+            grad_add_row(P.flags, g, cg, row, metallic_on ? 5 : 4);
+        }
+        __syncwarp(mask);
+        if (!__any_sync(mask, hits == 15u && r.tr > P.min_transmittance)) break;
+    }
+}
+
 }  // namespace ptir

@@ -1036,9 +1036,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_wb_bounce(TraceParams P, BwdInp
 
 template <int K>
 __global__ void __launch_bounds__(kMaxThreads) k_wb_replay(TraceParams P, BwdInputs B, WfView W, unsigned cursor,
-                                                           bool resume) {
+                                                           bool resume, unsigned quad_jobs) {
     PTIR_STAGE_PROLOGUE
     const unsigned count = W.count[kQJobs];
+    if (count <= quad_jobs) return;  // the quads' launch
     // with `resume` a replay's rounds after its first resume from the previous round's frontier
     const Frontier F{resume ? W.frontier + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2 * W.frontier_cap
                             : nullptr,
@@ -1051,6 +1052,84 @@ __global__ void __launch_bounds__(kMaxThreads) k_wb_replay(TraceParams P, BwdInp
             const ReplayJob j = W.jobs[i];
             replay_material_grad(C, B, j, F.buf ? &F : nullptr);
         }
+    }
+    flush_counters(P, ctr);
+}
+
+// k_wb_replay with resumed rounds (K <= 16) for up to kQuadRays jobs, a quad of lanes a job (quad.cuh): the entries
+// that a round sets aside come in the order of the one-lane replay, so the same hits are scattered with the same
+// weights. Bound, as there, by the latency of a step, of which a job is a chain. Replay stage, against one lane a job:
+// 3.1 -> 2.4 ms (80k paths, 20k Gaussians), 4.9 -> 3.3 (90k, 100k), 7.3 -> 5.9 (90k, 300k); with 786k paths over
+// 1M Gaussians it took 41 ms against 18.6 (twice the frontier traffic an issue slot), hence the line.
+template <int K>
+__global__ void __maxnreg__(128) k_wb_replay_quad(TraceParams P, BwdInputs B, WfView W, unsigned cursor, int refill,
+                                                 unsigned quad_jobs) {
+    extern __shared__ float4 quad_mem[];
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    enum : int { kIdle = 0, kTracing = 1, kReady = 2 };
+    const unsigned ln = lane(), c = ln & 3u, base = ln & 28u;
+    StackEntry* const stack = reinterpret_cast<StackEntry*>(quad_mem) + (threadIdx.x >> 2) * kQuadStackEntries;
+    TraceCounters ctr = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const unsigned count = W.count[kQJobs];
+    if (count > quad_jobs) return;
+    const bool in_use = (ln >> 2) < quads_in_use(count);
+    int phase = kIdle;
+    int rounds = 0;
+    bool drained = false;
+    ReplayState r;
+    QuadTrace<K> t;
+    t.tk = kFarT;
+    kbuf_clear(t.kt, t.kid);
+    QuadFrontier F{W.frontier + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 2) * 2 * W.frontier_cap, W.frontier_cap,
+                   0, 0, 0, 0};
+    // next round of the job, false when it is complete
+    auto next_round = [&]() -> bool {
+        if (!replay_open(P, r)) return false;
+        if (rounds > (1 << 16)) {
+            if (c == 0) atomicOr(P.error_word, kErrLoopBound);
+            return false;
+        }
+        const bool resume = rounds++ > 0;
+        phase = quad_start_resume(P.accel, r.o, r.d, r.start + 1e-9f, r.end, t, F, resume, ctr, c) ? kTracing : kReady;
+        return true;
+    };
+    while (true) {
+        const unsigned idle = __ballot_sync(kFull, phase == kIdle && in_use && c == 0);
+        if (!drained && idle) {
+            const unsigned n_idle = __popc(idle);
+            unsigned first = 0;
+            if (ln == 0) first = atomicAdd(W.cursor + cursor, n_idle);
+            first = __shfl_sync(kFull, first, 0);
+            drained = first + n_idle >= count;
+            const unsigned i = first + __popc(idle & ((1u << base) - 1u));
+            if (phase == kIdle && in_use && i < count) {
+                TraceCounters mine = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+                replay_begin(P, W.jobs[i], r, mine);
+                if (c == 0) ctr.replay += mine.replay;
+                rounds = 0;
+                if (!next_round()) phase = kIdle;
+            }
+        }
+        const unsigned busy = __ballot_sync(kFull, phase != kIdle && c == 0);
+        if (!busy) {
+            if (drained) break;
+            continue;
+        }
+        while (true) {
+            const unsigned tracing = __ballot_sync(kFull, phase == kTracing);
+            if (!tracing || __popc(busy) - (__popc(tracing) >> 2) >= (drained ? 1 : refill)) break;
+            if (phase == kTracing && !quad_step_resume<K>(P.accel, r.o, r.d, t, F, stack, P.error_word, ctr, ln, tracing))
+                phase = kReady;
+        }
+        __syncwarp();  // the entries set aside, before the next call reads them
+        const unsigned ready = __ballot_sync(kFull, phase == kReady);
+        if (phase == kReady) {
+            const float t_last = __shfl_sync(ready, t.kt[QuadTrace<K>::L - 1], base + 3u);
+            quad_replay_batch(P, B, r, t, ctr, ln, ready);
+            // a k-buffer that is not full held every candidate of the round
+            if (!(t_last < kFarT && next_round())) phase = kIdle;
+        }
+        __syncwarp();
     }
     flush_counters(P, ctr);
 }
@@ -1370,14 +1449,25 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
     const bool resume = use_resume<K>(tune);
     const bool resume_replay = K <= 16 && tune.resume_replay;
     const TraceLaunch trace0 = trace_launch<K, false, false>(tune, resume), trace = trace_launch<K, false, true>(tune, resume);
+    // replays with resumed rounds: a quad a job up to kQuadRays jobs (at most two a path), a lane a job above
+    const size_t quad_stacks = sizeof(StackEntry) * kQuadStackEntries * (size_t)(B / 4);
+    const unsigned quad_jobs = resume_replay ? kQuadRays : 0u;
+    const bool lane_jobs = 2ull * 32ull * chunk_tiles > quad_jobs;
     const int g_replay = grid_cached((const void*)k_wb_replay<K>, B);
-    const int g_front = std::max(resume ? std::max(trace0.lane_grid, trace.lane_grid) : 0, resume_replay ? g_replay : 0);
-    if (g_front > 0 && (e = frontier_reserve(b, (size_t)g_front * B, s)) != cudaSuccess) return e;
+    int g_replay_quad = 0;
+    if constexpr (K <= 16) {
+        if (resume_replay) g_replay_quad = grid_cached((const void*)k_wb_replay_quad<K>, B, quad_stacks);
+    }
+    // frontiers: one a thread of a resumed kernel, one a quad of the replay
+    const size_t fronts = std::max({resume ? (size_t)std::max(trace0.lane_grid, trace.lane_grid) * B : (size_t)0,
+                                    resume_replay && lane_jobs ? (size_t)g_replay * B : (size_t)0,
+                                    (size_t)g_replay_quad * B / 4});
+    if (fronts > 0 && (e = frontier_reserve(b, fronts, s)) != cudaSuccess) return e;
     const unsigned mb = p.render_opts ? std::min(p.max_bounces, 2u) : p.max_bounces;
     if (kFirstBounceCursor + 3u * mb > (unsigned)kNumCursors) return cudaErrorInvalidValue;
     for (unsigned long long t0 = 0; t0 < tiles; t0 += chunk_tiles) {
         const unsigned nt = (unsigned)std::min<unsigned long long>(chunk_tiles, tiles - t0);
-        const WfView W = view_of(b, t0, nt * 32u, g_front > 0);
+        const WfView W = view_of(b, t0, nt * 32u, fronts > 0);
         e = cudaMemsetAsync(b.counters, 0, sizeof(unsigned) * (kNumQueueCounts + kNumCursors), s);
         if (e != cudaSuccess) return e;
         const int cap = (int)std::min<long long>(INT32_MAX, ((long long)nt * 32 + B - 1) / B);
@@ -1404,7 +1494,14 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
             });
             ++cursor;
             sc.run(kStageReplay, p, s, [&](const TraceParams& q) {
-                k_wb_replay<K><<<g_replay, B, 0, s>>>(q, bi, W, cursor, resume_replay);
+                if constexpr (K <= 16) {
+                    if (resume_replay) {
+                        const long long need = (2ll * W.slots + B / 32 - 1) / (B / 32);
+                        k_wb_replay_quad<K><<<(unsigned)std::min<long long>(g_replay_quad, need), B, quad_stacks, s>>>(
+                            q, bi, W, cursor, (R + 7) / 8, quad_jobs);
+                    }
+                }
+                if (lane_jobs) k_wb_replay<K><<<g_replay, B, 0, s>>>(q, bi, W, cursor, resume_replay, quad_jobs);
             });
             ++cursor;
             if (depth + 1 >= mb) break;
