@@ -23,6 +23,7 @@
 
 #include "radix_sort.cuh"
 #include "path.cuh"
+#include "near.cuh"
 #include "quad_path.cuh"
 #include "wavefront.h"
 
@@ -247,9 +248,9 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
                                                       const unsigned* items, int out_q, unsigned cursor, int refill,
                                                       unsigned quad_rays) {
     constexpr bool kPair = K == 32;  // traversals gather two 16-candidate rounds (leaf-index k-buffer)
-    static_assert(!(kPair && kResume), "resumed calls take the 16-candidate rounds one by one");
+    // the k-buffer holds leaf record indices
+    static_assert(kPair != kResume, "rounds from the root with K <= 16 are k_wf_trace_near's and k_wf_trace_quad's");
     static_assert(!(kSlack && kResume), "the exact-candidate slack is applied by the rounds from the root");
-    constexpr bool kIdx = kPair || kResume;  // the k-buffer holds leaf record indices
     const int nthreads = (int)(gridDim.x * blockDim.x);
     const Frontier F{kResume ? W.frontier + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2 * W.frontier_cap
                              : nullptr,
@@ -270,18 +271,9 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
     bool drained = false;
     float3 ro = f3(0.0f), rd = f3(0.0f);  // the lane's segment ray
     TraceState t;
-    bool seeded = false;  // the lane's call started with a cut estimated from its previous round
-    float first_span = 0.0f;  // K-th distance less tmin of the first round of the lane's last segment
     float kt[K];  // a call found nothing when kt[0] == kFarT
     unsigned kid[K];
-    // next trace call of this lane's segment, or ready with nothing found when it is complete. The
-    // rounds of the reference's k-buffer of 16 (from the root) are seeded (traverse.cuh: a call that
-    // does not fill its k-buffer below its seed is continued past it): a segment's later round with
-    // the cut tmin + kSeedSpan x the previous round's span of distances, its first round with tmin +
-    // kSeedSpan x the first-round span (K-th distance less tmin) of the lane's last segment, a
-    // neighbouring ray in the queue's order. Rounds of 8 are not seeded: their spans are short, and
-    // a seed that close culls more grazing Gaussians (0.17 % of the paths changed on a scene of
-    // Gaussians up to 0.3 in size).
+    // next trace call of this lane's segment, or ready with nothing found when it is complete
     auto next_call = [&](const Composite& c) {
         if (!composite_open(P, c)) {
             kt[0] = kFarT;
@@ -294,19 +286,8 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
             phase = kReady;
             return;
         }
-        float cap = kFarT;
-        seeded = false;
-        if constexpr (!kIdx && K == 16) {
-            // kt still holds the previous round (a full k-buffer) when there is one
-            const float span = rounds > 1 ? kt[K - 1] - kt[0] : first_span;
-            if (span > 0.0f) {
-                cap = composite_tmin(c) + kSeedSpan * span;
-                seeded = cap < composite_tend(c);
-                if (!seeded) cap = kFarT;
-            }
-        }
-        phase = trace_start<K, kIdx, kResume>(P.accel, ro, rd, composite_tmin(c), composite_tend(c), kt, kid, t, ctr,
-                                              &F, rounds > 1, cap)
+        phase = trace_start<K, true, kResume>(P.accel, ro, rd, composite_tmin(c), composite_tend(c), kt, kid, t, ctr, &F,
+                                              rounds > 1)
                     ? kTracing
                     : kReady;
     };
@@ -350,15 +331,8 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
             const unsigned tracing = __ballot_sync(kFull, phase == kTracing);
             if (!tracing || __popc(eligible & ~tracing) >= refill) break;
             if (phase == kTracing &&
-                !trace_step<K, kIdx, kResume, kSlack>(P.accel, ro, rd, t, kt, kid, stack, P.error_word, ctr,
-                                                      &F)) {
-                if (seeded && kid[K - 1] == kNoHit) {
-                    seeded = false;
-                    trace_continue(t, kt, ctr);
-                } else {
-                    phase = kReady;
-                }
-            }
+                !trace_step<K, true, kResume, kSlack>(P.accel, ro, rd, t, kt, kid, stack, P.error_word, ctr, &F))
+                phase = kReady;
         }
         // composite the finished calls; hand on the finished segments
         bool done = false;
@@ -393,18 +367,139 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
                     if (call) next_call(c);
                     else no_call();
                 } else {
-                    if constexpr (kIdx)
-                        composite_leaf_batch<kSelfOcc>(P, ctr, c, batch_t, batch_id, nthreads, 0, K, mark);
-                    else
-                        composite_hits_strided<kSelfOcc, K>(P, ctr, c, batch_t, batch_id, nthreads, mark);
+                    composite_leaf_batch<kSelfOcc>(P, ctr, c, batch_t, batch_id, nthreads, 0, K, mark);
                     // a k-buffer that is not full held every candidate of the call: a later call finds none
-                    if (rounds == 1 && kid[K - 1] != kNoHit) first_span = kt[K - 1] - t.tmin;
                     if (kid[K - 1] != kNoHit) next_call(c);
                     else no_call();
                 }
             }
             // nothing found, segment closed, or loop bound: the segment is complete
             if (phase == kReady && kt[0] >= kFarT) {
+                Segment s;
+                Pcg32 rng = load_rng(W, q);
+                composite_end(P, c, W.seg[q].scatter_pdf, W.seg[q].light_pdf, s, rng);
+                W.seg[q] = s;
+                store_rng(W, q, rng);
+                phase = kIdle;
+                done = true;
+            } else {
+                pk.save(c);
+            }
+        }
+        if (out_q >= 0) push(W.q[out_q], W.count + out_q, q, done);
+    }
+    flush_counters(P, ctr);
+}
+
+// k_wf_trace for the rounds from the root (K <= 16), with the k-buffer of near.cuh: the same calls, seeds and
+// compositing. 72 registers: on 786k paths over 1M Gaussians (forward and adjoint) the stage took 135.3 ms, against
+// 139.2 at 80, 151.1 at 64 and 178.0 at 56.
+template <int K, bool kMark, bool kSelfOcc, bool kSlack>
+__global__ void __maxnreg__(72) k_wf_trace_near(TraceParams P, float* vis, WfView W, int in_q, const unsigned* items,
+                                                int out_q, unsigned cursor, int refill, unsigned quad_rays) {
+    const int nthreads = (int)(gridDim.x * blockDim.x);
+    float* const base = W.parked + blockIdx.x * blockDim.x + threadIdx.x;
+    const Parked pk{base, nthreads};
+    float* const batch_t = base + kParkedFields * nthreads;
+    unsigned* const batch_id = reinterpret_cast<unsigned*>(batch_t + K * nthreads);
+    StackEntry stack[kStackDepth];
+    uint2 log[kNearLog];
+    TraceCounters ctr = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    enum : int { kIdle = 0, kTracing = 1, kReady = 2 };
+    const unsigned count = W.count[in_q];
+    if (count <= quad_rays) return;  // the quads' launch
+    int phase = kIdle;
+    unsigned q = 0;
+    int rounds = 0;
+    bool drained = false, seeded = false;
+    float3 ro = f3(0.0f), rd = f3(0.0f);
+    TraceState t;
+    float first_span = 0.0f;
+    Near<K> b;
+    near_clear(b);
+    // next trace call of this lane's segment, or ready with nothing found when it is complete
+    auto next_call = [&](const Composite& c) {
+        // kt still holds the previous round (a full k-buffer) when there is one
+        const float span = rounds > 0 ? b.kt[K - 1] - b.kt[0] : first_span;
+        phase = kReady;
+        bool call = composite_open(P, c);
+        if (call && ++rounds > kMaxRounds + 1) {
+            atomicOr(P.error_word, kErrLoopBound);
+            call = false;
+        }
+        if (!call) {
+            b.kt[0] = kFarT;
+            return;
+        }
+        float cap = kFarT;
+        seeded = false;
+        if (K == 16 && span > 0.0f) {
+            cap = composite_tmin(c) + kSeedSpan * span;
+            seeded = cap < composite_tend(c);
+            if (!seeded) cap = kFarT;
+        }
+        if (near_start<K>(P.accel, ro, rd, composite_tmin(c), composite_tend(c), b, log, t, ctr, cap)) phase = kTracing;
+    };
+    while (true) {
+        // refill the idle lanes
+        const unsigned idle = __ballot_sync(kFull, phase == kIdle);
+        if (!drained && idle) {
+            const unsigned n_idle = __popc(idle);
+            unsigned first = 0;
+            if (lane() == 0) first = atomicAdd(W.cursor + cursor, n_idle);
+            first = __shfl_sync(kFull, first, 0);
+            drained = first + n_idle >= count;
+            if (phase == kIdle) {
+                const unsigned i = first + __popc(idle & lanes_below());
+                if (i < count) {
+                    q = items[i];
+                    Composite c;
+                    composite_begin(P, c, W.seg[q].o, W.seg[q].d);
+                    ro = c.o;
+                    rd = c.d;
+                    ++ctr.segments;
+                    rounds = 0;
+                    next_call(c);
+                    pk.save(c);
+                }
+            }
+        }
+        const unsigned busy = __ballot_sync(kFull, phase != kIdle);
+        if (!busy) {
+            if (drained) break;
+            continue;
+        }
+        // traverse until enough lanes wait
+        const unsigned eligible = drained ? busy : kFull;
+        while (true) {
+            const unsigned tracing = __ballot_sync(kFull, phase == kTracing);
+            if (!tracing || __popc(eligible & ~tracing) >= refill) break;
+            if (phase == kTracing && !near_step<K, kSlack>(P.accel, ro, rd, t, b, log, stack, P.error_word, ctr)) {
+                if (seeded && b.kt[K - 1] >= kFarT) {
+                    seeded = false;
+                    trace_continue(t, b.kt, ctr);
+                } else {
+                    phase = kReady;
+                }
+            }
+        }
+        // composite the finished calls; hand on the finished segments
+        bool done = false;
+        if (phase == kReady) {
+            Composite c;
+            pk.load(c, ro, rd);
+            if (b.kt[0] < kFarT) {
+                near_resolve(b, log, batch_t, batch_id, nthreads);
+                composite_hits_strided<kSelfOcc, K>(P, ctr, c, batch_t, batch_id, nthreads, kMark ? vis : nullptr);
+                const bool full = b.kt[K - 1] < kFarT;
+                if (rounds == 1 && full) first_span = b.kt[K - 1] - t.tmin;
+                // a k-buffer that is not full held every candidate of the call: a later call finds none
+                if (full) next_call(c);
+                else b.kt[0] = kFarT;
+            }
+            // nothing found, segment closed, or loop bound: the segment is complete
+            if (phase == kReady && b.kt[0] >= kFarT) {
                 Segment s;
                 Pcg32 rng = load_rng(W, q);
                 composite_end(P, c, W.seg[q].scatter_pdf, W.seg[q].light_pdf, s, rng);
@@ -1318,7 +1413,7 @@ static bool use_resume(const WavefrontTuning& tune) {
 
 // An intersection launch: the kernels of its k-buffer size and options, and their persistent grids. Rounds from
 // the root with K <= 16 take four lanes a ray (k_wf_trace_quad) in a launch of up to kQuadRays rays and one lane
-// a ray (k_wf_trace) in a larger one; resumed rounds and K = 32 always take one.
+// a ray (k_wf_trace_near) in a larger one; resumed rounds and K = 32 take one (k_wf_trace).
 struct TraceLaunch {
     const void* lane_fn = nullptr;
     const void* quad_fn = nullptr;
@@ -1336,8 +1431,8 @@ static TraceLaunch trace_launch(const WavefrontTuning& tune, bool resume) {
         if (resume) {
             l.lane_fn = (const void*)k_wf_trace<K, kMark, kSelfOcc, true, false>;
         } else {
-            l.lane_fn = slack ? (const void*)k_wf_trace<K, kMark, kSelfOcc, false, true>
-                              : (const void*)k_wf_trace<K, kMark, kSelfOcc, false, false>;
+            l.lane_fn = slack ? (const void*)k_wf_trace_near<K, kMark, kSelfOcc, true>
+                              : (const void*)k_wf_trace_near<K, kMark, kSelfOcc, false>;
             l.quad_fn = slack ? (const void*)k_wf_trace_quad<K, kMark, kSelfOcc, true>
                               : (const void*)k_wf_trace_quad<K, kMark, kSelfOcc, false>;
         }
