@@ -214,7 +214,7 @@ def _clock_summary(lines: list):
 
 # ------------------------------------------------------------------------------------------
 STAGES = ("intersect", "shadow", "replay", "shading", "megakernel", "sort")
-KERNEL_OF_STAGE = {"intersect": "k_wf_trace", "shadow": "k_wf_shadow", "replay": "k_wb_replay",
+KERNEL_OF_STAGE = {"intersect": "k_wf_trace_near/quad", "shadow": "k_wf_shadow", "replay": "k_wb_replay",
                    "shading": "k_wf_camera/primary/bounce", "megakernel": "k_trace_fwd/k_trace_bwd",
                    "sort": "k_wf_sort_keys + radix sort"}
 ACCEL_KERNELS_PER_BUILD = 6  # the step's refit: k_prep, k_bounds_partial, k_bounds_final, k_gather, k_refit, k_emit4
@@ -317,9 +317,9 @@ def _view_config(views):
 # a material gradient, so the adjoint re-traverses those segments even where no light reaches the
 # camera (the 1M-Gaussian scene's opaque shell keeps its pbr image black).
 LOSS_L1, LOSS_ALBEDO, LOSS_ROUGHNESS = 0.8, 0.5, 0.2
-# dram__bytes_read.sum + dram__bytes_write.sum of k_wf_trace per segment it intersects, from an ncu
-# capture of 16 launches on 2 views of 512x384x4 (1,184,413,952 bytes over ~1,652,977 segments)
-DRAM_BYTES_PER_INTERSECT_SEGMENT = 716.5
+# dram__bytes_read.sum + dram__bytes_write.sum of the intersection kernels per segment they intersect, from
+# an ncu capture of a forward pass's launches on 2 views of 512x384x4 (5,223,165,184 bytes over 2,479,466 segments)
+DRAM_BYTES_PER_INTERSECT_SEGMENT = 2106.6
 STEP_DESC = ("lbvh refit + forward + loss (0.8 L1(pbr, target) + 0.5 L2(albedo, prior) + 0.2 L2(roughness, prior)) "
              "+ adjoint + selective adam (material, env)")
 

@@ -9,10 +9,11 @@
 //   4. sort      key/id radix sort (radix_sort.cuh: stable LSD, 8-bit digits)
 //   5. gather    leaf records in key order
 //   6. hierarchy internal nodes from the sorted keys (ties broken by position), or PLOC
-//                (agglomerative clustering by surface area over the sorted leaves)
+//                (agglomerative clustering by surface area over the sorted leaves: two launches an
+//                iteration, the last few thousand clusters in one block)
 //   7. refit     bottom-up child boxes with arrival counters
 //   8. collapse  4-wide nodes, greedy by surface area (rebuild only)
-//   9. emit      the 4-wide node records the traversal reads
+//   9. emit      the 4-wide node records the traversal reads, by rows (one lane a ray) and child by child (four)
 // A refit (rebuild == false, same n) redoes 1, 2, 5, 7 and 9 in the stored leaf order and topology.
 #include <algorithm>
 #include <cstring>
@@ -396,9 +397,9 @@ __device__ __forceinline__ bool ploc_before(const PlocPair& a, const PlocPair& b
 
 // The iterations from kPlocTail clusters to the root, in one block with the list in shared memory. Most of a build's
 // iterations are here: the last few thousand clusters merge a few pairs at a time (a million Gaussians take about
-// 70 iterations to 3000 clusters and 60 from there), and as launches each cost four kernels of a few us and a
-// quarter of a host round trip. As many lanes as fit share the search of a cluster's 32 neighbours; the
-// order of pairs is strict, so the pairs are those of k_ploc_pair. Bound by the latency of the
+// 70 iterations to 3000 clusters and 60 from there), and as launches each cost kernels of a few us (four when
+// this was measured, two now) and a quarter of a host round trip. As many lanes as fit share the search of a
+// cluster's 32 neighbours; the order of pairs is strict, so the pairs are those of k_ploc_pair. Bound by the latency of the
 // iteration (search, merge, scan): a rebuild of a million Gaussians took 10.75 ms and takes 4.3 with this kernel,
 // the collapse in parallel (k_collapse_level) and the scratch kept.
 struct PlocTail {

@@ -7,9 +7,9 @@
 
 namespace ptir {
 
-// Acceleration structure over the Gaussians' instance boxes. The LBVH is built binary and
-// traversed 4-wide: every binary node at even depth becomes a 4-wide node holding the boxes of
-// its (up to four) grandchildren, so one 128-byte fetch tests four boxes.
+// Acceleration structure over the Gaussians' instance boxes. The hierarchy is built binary
+// and traversed 4-wide: a 4-wide node holds the boxes of up to four descendants of a binary node (greedy by
+// surface area), so one 128-byte fetch tests four boxes.
 //   node4 = 8 x float4: lo.x[4] lo.y[4] lo.z[4] hi.x[4] hi.y[4] hi.z[4] child[4] kmax[4]
 //           (kmax: the largest kernel support radius of any Gaussian under the child);
 //           a child c >= 0 is a 4-wide node, kNoChild an empty slot, any other c < 0 leaf ~c.

@@ -7,7 +7,7 @@
 // instructions an entry), every inserted (distance, id) is appended to a log in local memory, and the ids
 // are put in order once, when the call ends (near_resolve). With 16 registers less the kernel fits 72, seven blocks
 // of 128 threads an SM instead of five. Intersection stage of 786k paths over 1M Gaussians, forward and
-// adjoint: 147.5 -> 135.3 ms; of 500k over 600k: 72.3 -> 68.2.
+// adjoint: 147.5 -> 135.3 ms; of 627k over 600k: 72.3 -> 68.2.
 #pragma once
 
 #include "leaf.cuh"

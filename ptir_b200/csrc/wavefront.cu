@@ -7,13 +7,15 @@
 //   primary  : primary outputs, NEE light sample                       -> shadow queue | bounce queue
 //   shadow   : stochastic shadow ray of the NEE sample                -> bounce queue
 //   bounce d : light gathering, path termination, BRDF sample          -> intersect queue
-//   sort     : the intersect queue in (octant, origin cell, direction cell) order
+//   sort     : the intersect queue in (octant, origin cell, direction cell) order, where it holds more than
+//              kQuadRays rays
 //   intersect: next segment                                            -> bounce queue
 // and the backward the same with the adjoint stages, whose re-traversals (the reference's
 // rayIntersectBwd) go to a replay queue drained after every bounce stage. Path state lives in
 // HBM between stages; queues are appended with one atomic per warp (ballot + popc). The
-// intersect stage refills lanes one by one (k_wf_trace). The per-path order of random draws is
-// the megakernel's, so both schedules produce the same paths.
+// intersect, shadow and replay stages take four lanes a ray for queues of up to kQuadRays (quad.cuh) and
+// one lane a ray above; the queue's count on the device decides. Lanes and quads are refilled one by one.
+// The per-path order of random draws is the megakernel's, so both schedules produce the same paths.
 
 #include <algorithm>
 #include <cstdint>
@@ -210,11 +212,15 @@ struct Parked {
 // The warp leaves its traversal loop once `refill` lanes wait (a finished call, or idle while
 // the queue still holds segments). W.parked holds, per thread of the grid, the parked
 // accumulators and, while a batch is composited, its k-buffer (kParkedFields + 2K floats).
+//
+// Three kernels do this: k_wf_trace (two rounds a traversal with K = 32, and resumed rounds), k_wf_trace_near
+// (rounds from the root, K <= 16) and k_wf_trace_quad (the same, four lanes a ray, for small launches).
+//
 // Registers per thread of k_wf_trace (and of the shadow kernel of the same k-buffer size). The
 // kernels use no shared memory, so registers alone set the resident warps. K <= 16: 96, five
 // 128-thread blocks per SM, 5 % faster than the compiler's own 127 (four blocks) despite a few
-// spills; 80 (six blocks) was 11 % slower. K = 32: 128, four blocks, 6 % faster for the step
-// than 168 (three blocks); 96 (five blocks) was 23 % slower.
+// spills; 80 (six blocks) was 11 % slower (both measured on rounds from the root).
+// K = 32: 128, four blocks, 6 % faster for the step than 168 (three blocks); 96 (five blocks) was 23 % slower.
 constexpr int trace_regs(int K) { return K > 16 ? 128 : 96; }
 
 // Seed of the k-buffer rounds in the intersection stage: the cut starts at the round's tmin plus
@@ -225,10 +231,11 @@ constexpr int trace_regs(int K) { return K > 16 ? 128 : 96; }
 // of them continued), against 145.5 ms at 1.5 and 143.2 ms at 3.
 constexpr float kSeedSpan = 2.0f;
 
-// Rays up to which an intersection launch takes four lanes a ray. Measured against one lane (intersection stage,
-// ms): 1.93 -> 0.93 at 16k rays over 10k Gaussians, 36.2 -> 23.3 at 90k over 300k, 9.3 -> 7.7 at 278k
-// primary and 80k bounce rays over 30k; all of a launch of 786k primary and about 200k bounce rays over 1M
-// took 157.6 against 147.8, and with the line at 262,144 instead of 131,072 150.4.
+// Rays up to which an intersection launch takes four lanes a ray. Measured against one lane (the stage, ms):
+// 1.93 -> 0.93 at 16k rays over 10k Gaussians, 36.2 -> 23.3 at 90k over 300k. Where the line lies, against
+// k_wf_trace_near (lines at 65,536 / 94,720 / 131,072 / 262,144 rays): 8.0 / 7.9 / 7.5 / 7.5 at 278k primary
+// and 80k bounce rays over 30k Gaussians; 67.8 / 67.7 / 68.8 / 73.5 at 627k paths of several views over 600k;
+// 135.0 / 135.6 / 135.0 / 142.0 at 786k primary and about 200k bounce rays over 1M.
 constexpr unsigned kQuadRays = 1u << 17;
 
 //
@@ -537,8 +544,8 @@ PTIR_DEV unsigned quads_in_use(unsigned count) {
     return min(8u, max(1u, (count + warps - 1u) / warps));
 }
 
-// k_wf_trace for the rounds from the root (K <= 16) of small launches, a quad of lanes per segment (quad.cuh).
-// The decisions, their order and the compositing are k_wf_trace's, and no first round is seeded: a quad rarely
+// The rounds from the root (K <= 16) of small launches, a quad of lanes per segment (quad.cuh).
+// The decisions, their order and the compositing are k_wf_trace_near's, and no first round is seeded: a quad rarely
 // sees more than a few segments. A small launch is bound by the chain of its slowest ray, which one lane walks
 // at about 1 us a visit; here the visit's parts run side by side (preview of 2,867 rays over 2k Gaussians:
 // 1.42 -> 0.49 ms in the stage). 96 registers hold the visit without spills: 23.6 ms at 90k rays over 300k

@@ -22,11 +22,11 @@ struct WavefrontBuffers {
     void* jobs = nullptr;    // ReplayJob[2 * slots]
     void* counters = nullptr;  // u32[kNumQueueCounts + kNumCursors]
     void* sort_keys[2] = {nullptr, nullptr};  // u32[slots]: ray-order keys, unsorted and sorted
-    void* sorted = nullptr;  // u32[slots]: the intersect queue in key order
+    void* sorted = nullptr;  // u32[slots]: a queue in key order (queues of more rays than the quads take)
     void* sort_temp = nullptr;
     size_t sort_temp_bytes = 0;
-    void* parked = nullptr;  // f32, per resident thread of the intersection kernel (k_wf_trace)
-    void* frontier = nullptr;  // uint2[2 * kFrontierCap] per thread of the intersection kernel
+    void* parked = nullptr;  // f32, per resident thread of the one-lane intersection kernels
+    void* frontier = nullptr;  // uint2[2 * kFrontierCap] per thread (quad) of a kernel with resumed rounds
     size_t frontier_threads = 0;
 };
 
@@ -48,7 +48,7 @@ struct WavefrontTuning {
     int kbuf = 16;                  // candidates per traversal: 8, 16 or 32
     int refill_lanes = 32;          // intersection: waiting lanes (1..32) before a warp refills
     int block = 128;                // threads per block: 64, 128 or 256
-    bool sort_rays = true;          // intersect bounce rays in (octant, origin cell, direction cell) order
+    bool sort_rays = true;          // bounce and shadow queues of one lane a ray in (octant, origin cell, direction cell) order
     int shadow_kbuf = 16;           // candidates per shadow-ray traversal: 8, 16 or 32
     bool resume_isect = false;      // intersection stage: rounds resumed from the previous round's frontier (K <= 16)
     bool resume_replay = true;      // backward replay: the same
