@@ -16,6 +16,7 @@ namespace ptir {
 
 // Log entries a lane, (distance bits, id) in insertion order. A full log drops what is past the K-th
 // distance: that leaves at most K - 1 nearer entries and K equal ones.
+// A call of 16 inserts about 34 entries. 34 entries of log: 136.5 ms in the stage at 1M Gaussians; 48: 135.0; 64: 134.7.
 constexpr int kNearLog = 48;
 
 template <int K>
