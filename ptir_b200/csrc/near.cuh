@@ -7,7 +7,8 @@
 // instructions an entry), every inserted (distance, id) is appended to a log in local memory, and the ids
 // are put in order once, when the call ends (near_resolve). With 16 registers less the kernel fits 72, seven blocks
 // of 128 threads an SM instead of five. Intersection stage of 786k paths over 1M Gaussians, forward and
-// adjoint: 147.5 -> 135.3 ms; of 627k over 600k: 72.3 -> 68.2.
+// adjoint: 147.5 -> 133.0 ms; of 627k over 600k: 72.4 -> 66.3. (With the children sorted by integer keys that hold the
+// child in their two lowest bits, in place of descend's whole keys: 135.1 and 67.8, and another order of close keys.)
 #pragma once
 
 #include "leaf.cuh"
@@ -143,50 +144,7 @@ PTIR_DEV bool near_step(const AccelView& A, float3 o, float3 d, TraceState& t, N
         if (leaf_candidate_wide(A, ~c, o, d, t.tmin, t.tend, fminf(b.kt[K - 1], t.cap), ts, id, t.floor))
             near_insert(b, log, ts, id);
     }
-    // descent (descend): the children sorted by key as integers (keys are not negative), the child in the lowest two
-    // bits
-    const float cut = fminf(b.kt[K - 1], t.cap);
-    int s[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const bool in = ((v.hits >> k) & 1u) && v.ch[k] >= 0 && v.t0[k] <= cut;
-        s[k] = in ? (int)((__float_as_uint(v.key[k]) & ~3u) | (unsigned)k) : 0x7FFFFFFF;
-    }
-    auto order = [](int& x, int& y) {
-        const int lo = min(x, y), hi = max(x, y);
-        x = lo;
-        y = hi;
-    };
-    order(s[0], s[1]);
-    order(s[2], s[3]);
-    order(s[0], s[2]);
-    order(s[1], s[3]);
-    order(s[1], s[2]);
-    auto child_of = [&](int k) { return k == 0 ? v.ch[0] : (k == 1 ? v.ch[1] : (k == 2 ? v.ch[2] : v.ch[3])); };
-    if (s[0] != 0x7FFFFFFF) {
-        int sp = t.sp;
-#pragma unroll
-        for (int i = 3; i > 0; --i) {
-            if (s[i] == 0x7FFFFFFF) continue;
-            if (sp >= kStackDepth) {
-                atomicOr(err, kErrStackOverflow);
-                ctr.candidates += kbuf_count(b.kt);
-                return false;
-            }
-            const int k = s[i] & 3;
-            stack[sp++] = make_int2(child_of(k), __float_as_int(k == 0 ? v.t0[0] : (k == 1 ? v.t0[1] : (k == 2 ? v.t0[2] : v.t0[3]))));
-        }
-        t.sp = sp;
-        t.node = child_of(s[0] & 3);
-        return true;
-    }
-    while (t.sp > 0) {
-        const StackEntry e = stack[--t.sp];
-        if (__int_as_float(e.y) <= cut) {
-            t.node = e.x;
-            return true;
-        }
-    }
+    if (descend<K>(t, v, b.kt, stack, err, ctr)) return true;
     ctr.candidates += kbuf_count(b.kt);
     return false;
 }

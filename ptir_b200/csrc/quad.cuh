@@ -109,6 +109,26 @@ PTIR_DEV void quad_continue(QuadTrace<K>& t, TraceCounters& ctr) {
     t.sp = 0;
 }
 
+// descend's order (traverse.cuh) over a node's children, of which lane c holds child c, `inner` when it is an internal
+// one to be visited, and its key. The nearest is visited next, the lowest child of equal keys; the others are
+// stacked largest key first, the lowest child first of equal keys. Returns the number of stacked children, -1 when
+// there is no internal child; `best`: the next child's lane in the quad; `at`: a stacked child's place above the
+// stack's top. A key comes from an interval a <= b with a above 0, so it is no NaN and compares as an integer.
+// (Of equal keys those of lower children: c ^ 1 is lower where c is odd, c ^ 2 and c ^ 3 where c > 1; and the next
+// child, where its key is the lane's own, is not stacked.) Integer keys with the lane in their two lowest bits took
+// 4 % less of the stage (23.9 against 24.8 ms at 90k rays over 300k Gaussians), but they order keys that are equal or
+// within four units of the last place otherwise than descend.
+PTIR_DEV int quad_order(bool inner, float key, unsigned c, unsigned base, unsigned mask, unsigned& best, int& at) {
+    const int ik = inner ? __float_as_int(key) : 0x7FFFFFFF;
+    const int k1 = __shfl_xor_sync(mask, ik, 1), k2 = __shfl_xor_sync(mask, ik, 2), k3 = __shfl_xor_sync(mask, ik, 3);
+    const int least = min(min(ik, k1), min(k2, k3));
+    best = __ffs((__ballot_sync(mask, ik == least) >> base) & 15u) - 1;
+    const int i1 = ik - (int)(c & 1u), i2 = ik - (int)((c >> 1) & 1u);
+    const int np = __popc((__ballot_sync(mask, inner) >> base) & 15u) - 1;
+    at = np - 3 + (k1 > i1 ? 1 : 0) + (k2 > i2 ? 1 : 0) + (k3 > i2 ? 1 : 0) - (ik == least ? 1 : 0);
+    return np;
+}
+
 // One node visit of the quads in `mask` (whole quads, all of them tracing). Returns false when the
 // quad's call is complete. `stack` is the quad's, in shared memory.
 template <int K, bool kSlack>
@@ -153,23 +173,19 @@ PTIR_DEV bool quad_step(const AccelView& A, float3 o, float3 d, QuadTrace<K>& t,
         t.tk = __shfl_sync(mask, t.kt[L - 1], base + 3u);
         cut = fminf(t.tk, t.cap);
     }
-    // descent: the internal children still in front of the cut, nearest key first; the others are stacked
-    // largest key first. Keys are compared as integers (they are not negative) with the child in the two
-    // lowest bits, so that they differ and name their lane.
+    // descent: the internal children still in front of the cut
     const bool inner = hit && child >= 0 && t0 <= cut;
-    const int ik = inner ? (int)((__float_as_uint(key) & ~3u) | c) : 0x7FFFFFFF;
-    const int k1 = __shfl_xor_sync(mask, ik, 1), k2 = __shfl_xor_sync(mask, ik, 2), k3 = __shfl_xor_sync(mask, ik, 3);
-    const int rank = (k1 < ik ? 1 : 0) + (k2 < ik ? 1 : 0) + (k3 < ik ? 1 : 0);
-    const int best = min(min(ik, k1), min(k2, k3));
-    const int np = __popc((__ballot_sync(mask, inner) >> base) & 15u) - 1;  // stacked children
-    const int next = __shfl_sync(mask, child, base + (best & 3));
+    unsigned best;
+    int at;
+    const int np = quad_order(inner, key, c, base, mask, best, at);
+    const int next = __shfl_sync(mask, child, base + best);
     bool more = true, pop = np < 0;
     if (!pop) {
         if (t.sp + np > kStackDepth) {
             if (c == 0) atomicOr(err, kErrStackOverflow);
             more = false;
         } else {
-            if (inner && rank > 0) stack[t.sp + np - rank] = make_int2(child, __float_as_int(t0));
+            if (inner && c != best) stack[t.sp + at] = make_int2(child, __float_as_int(t0));
             t.sp += np;
             t.node = next;
         }
@@ -341,19 +357,17 @@ PTIR_DEV bool quad_step_resume(const AccelView& A, float3 o, float3 d, QuadTrace
     const bool child_in = hit && child >= 0;
     const bool inner = child_in && t0 <= t.tk;
     quad_defer(F, child_in && !inner, child, t0, c, base, mask);  // passed over after the leaf tests
-    const int ik = inner ? (int)((__float_as_uint(key) & ~3u) | c) : 0x7FFFFFFF;
-    const int k1 = __shfl_xor_sync(mask, ik, 1), k2 = __shfl_xor_sync(mask, ik, 2), k3 = __shfl_xor_sync(mask, ik, 3);
-    const int rank = (k1 < ik ? 1 : 0) + (k2 < ik ? 1 : 0) + (k3 < ik ? 1 : 0);
-    const int best = min(min(ik, k1), min(k2, k3));
-    const int np = __popc((__ballot_sync(mask, inner) >> base) & 15u) - 1;
-    const int next = __shfl_sync(mask, child, base + (best & 3));
+    unsigned best;
+    int at;
+    const int np = quad_order(inner, key, c, base, mask, best, at);
+    const int next = __shfl_sync(mask, child, base + best);
     bool more = true, pop = np < 0;
     if (!pop) {
         if (t.sp + np > kStackDepth) {
             if (c == 0) atomicOr(err, kErrStackOverflow);
             more = false;
         } else {
-            if (inner && rank > 0) stack[t.sp + np - rank] = make_int2(child, __float_as_int(t0));
+            if (inner && c != best) stack[t.sp + at] = make_int2(child, __float_as_int(t0));
             t.sp += np;
             t.node = next;
         }
