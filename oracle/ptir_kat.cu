@@ -2,12 +2,14 @@
 // known-answer entry points as the reference's kernels of oracle/ref_device_kat.cu: one thread per
 // case, inputs [n, IN] and outputs [n, OUT] floats in the same layouts, so that
 // tests/test_gpu_device_kat.py can run both on the cases of tests/golden/device_kat.npz. Also the
-// tracer's radix sort on device buffers (tests/test_gpu_sort.py). Built by `make -C oracle` with
-// the library's own nvcc flags.
+// tracer's radix sort on device buffers (tests/test_gpu_sort.py) and its k-buffers
+// (tests/test_gpu_kbuffer.py). Built by `make -C oracle` with the library's own nvcc flags.
 #include <cmath>
 #include <cstring>
 
+#include "../ptir_b200/csrc/near.cuh"
 #include "../ptir_b200/csrc/path.cuh"
+#include "../ptir_b200/csrc/quad.cuh"
 #include "../ptir_b200/csrc/radix_sort.cuh"
 
 namespace {
@@ -145,6 +147,69 @@ __global__ void k_light_pdf(int n, const float* in, float* out, TraceParams P) {
     out[i] = light_sampler_pdf(P, in3(a), in3(a + 3));
 }
 
+// The k-buffer after m insertions a case, as a traversal makes them (only what is nearer than the K-th distance),
+// and with `ev` what each insertion pushed out (id kNoHit: nothing). form 0: kbuf_insert_evict, one lane a case;
+// 1: quad_insert and 2: quad_insert_evict, four lanes; 3: near_insert and near_resolve, one lane.
+template <int K>
+__global__ void k_kbuffer(int form, int cases, int m, const float* ts, const unsigned* ids, float* out_t, unsigned* out_id,
+                          unsigned* ev) {
+    const int thread = blockIdx.x * blockDim.x + threadIdx.x;
+    if (form == 0 || form == 3) {
+        if (thread >= cases) return;
+        const float* t = ts + (size_t)thread * m;
+        const unsigned* id = ids + (size_t)thread * m;
+        if (form == 0) {
+            float kt[K];
+            unsigned kid[K];
+            kbuf_clear(kt, kid);
+            for (int i = 0; i < m; ++i) {
+                float et;
+                unsigned eid = kNoHit;
+                if (t[i] < kt[K - 1]) kbuf_insert_evict(kt, kid, t[i], id[i], et, eid);
+                ev[(size_t)thread * m + i] = eid;
+            }
+            for (int k = 0; k < K; ++k) {
+                out_t[(size_t)thread * K + k] = kt[k];
+                out_id[(size_t)thread * K + k] = kid[k];
+            }
+        } else {
+            Near<K> b;
+            uint2 log[kNearLog];
+            near_clear(b);
+            for (int i = 0; i < m; ++i)
+                if (t[i] < b.kt[K - 1]) near_insert(b, log, t[i], id[i]);
+            near_resolve(b, log, out_t + (size_t)thread * K, out_id + (size_t)thread * K, 1);
+        }
+        return;
+    }
+    constexpr int L = QuadTrace<K>::L;
+    const unsigned c = threadIdx.x & 3u, base = threadIdx.x & 28u;
+    const int at = thread >> 2;
+    const bool live = at < cases;
+    QuadTrace<K> q;
+    q.tk = kFarT;
+    kbuf_clear(q.kt, q.kid);
+    for (int i = 0; i < m; ++i) {
+        const float t = live ? ts[(size_t)at * m + i] : kFarT;
+        const unsigned id = live ? ids[(size_t)at * m + i] : kNoHit;
+        const float in = t < q.tk ? t : kFarT;
+        if (form == 1) {
+            quad_insert(q, in, id, c, 0xFFFFFFFFu);
+        } else {
+            float et;
+            unsigned eid;
+            quad_insert_evict(q, in, id, c, base, 0xFFFFFFFFu, et, eid);
+            if (live && c == 0) ev[(size_t)at * m + i] = eid;
+        }
+        q.tk = __shfl_sync(0xFFFFFFFFu, q.kt[L - 1], base + 3u);
+    }
+    if (!live) return;
+    for (int j = 0; j < L; ++j) {
+        out_t[(size_t)at * K + c * L + j] = q.kt[j];
+        out_id[(size_t)at * K + c * L + j] = q.kid[j];
+    }
+}
+
 int finish() { return cudaDeviceSynchronize() == cudaSuccess ? 0 : 1; }
 unsigned blocks(int n) { return (unsigned)((n + 127) / 128); }
 
@@ -233,6 +298,15 @@ int ptirkat_light_sample(int n, const float* in, float* out) {
 }
 int ptirkat_light_pdf(int n, const float* in, float* out) {
     k_light_pdf<<<blocks(n), 128>>>(n, in, out, g_params);
+    return finish();
+}
+
+// the k-buffer of `k` entries (8 or 16) in one of its forms (k_kbuffer) over `cases` sequences of m insertions
+int ptirkat_kbuffer(int k, int form, int cases, int m, const float* ts, const unsigned* ids, float* out_t, unsigned* out_id,
+                    unsigned* ev) {
+    const unsigned grid = blocks(form == 1 || form == 2 ? 4 * cases : cases);
+    if (k == 8) k_kbuffer<8><<<grid, 128>>>(form, cases, m, ts, ids, out_t, out_id, ev);
+    else k_kbuffer<16><<<grid, 128>>>(form, cases, m, ts, ids, out_t, out_id, ev);
     return finish();
 }
 
