@@ -310,9 +310,9 @@ PTIR_DEV bool quad_start_resume(const AccelView& A, float3 o, float3 d, float tm
     return true;
 }
 
-// One step of a resumable call (trace_step<K, true, true>) of the quads in `mask`: a node visit, or up to four
+// One step of a resumable call (trace_step<K, true, true, kSlack>) of the quads in `mask`: a node visit, or up to four
 // consecutive leaves of the frontier. The k-buffer holds leaf record indices. False when the call is complete.
-template <int K>
+template <int K, bool kSlack>
 PTIR_DEV bool quad_step_resume(const AccelView& A, float3 o, float3 d, QuadTrace<K>& t, QuadFrontier& F, StackEntry* stack,
                                unsigned* err, TraceCounters& ctr, unsigned ln, unsigned mask) {
     constexpr int L = QuadTrace<K>::L;
@@ -339,7 +339,7 @@ PTIR_DEV bool quad_step_resume(const AccelView& A, float3 o, float3 d, QuadTrace
                               fmaxf(fmaf(pz ? p.z : q.y, inv.z, -oi.z), t.tmin));
         const float b = min3f(fmaf(px ? p.w : p.x, inv.x, -oi.x), fmaf(py ? q.x : p.y, inv.y, -oi.y),
                               fminf(fmaf(pz ? q.y : p.z, inv.z, -oi.z), t.tend));
-        t0 = a;
+        t0 = (kSlack && t.slack > 0.0f) ? a - q.w * t.slack : a;
         key = 15.0f * a + b;
         crossed = child != kNoChild && a <= b;
         if (c == 0) ++ctr.nodes;

@@ -895,8 +895,9 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_shadow(TraceParams P, WfView W, 
 
 // k_wf_shadow for small launches, a quad of lanes a ray (quad.cuh): the same candidates, walked in the same order with
 // the same draws; no first round is seeded, as in k_wf_trace_quad. As there a small launch waits for its slowest
-// ray: stage of 16k rays over 10k Gaussians 0.60 -> 0.26 ms, of 90k over 300k (forward and adjoint) 6.6 -> 3.6 ms.
-template <int K>
+// ray: stage of 16k rays over 10k Gaussians 0.60 -> 0.26 ms, of 90k over 300k (forward and adjoint) 6.6 -> 4.1 ms.
+// kSlack: with the exact-candidate cull slack.
+template <int K, bool kSlack>
 __global__ void __maxnreg__(96) k_wf_shadow_quad(TraceParams P, WfView W, int refill, const unsigned* items,
                                                  unsigned quad_rays) {
     extern __shared__ float4 quad_mem[];
@@ -969,7 +970,7 @@ __global__ void __maxnreg__(96) k_wf_shadow_quad(TraceParams P, WfView W, int re
         while (true) {
             const unsigned tracing = __ballot_sync(kFull, phase == kTracing && !done);
             if (!tracing || __popc(busy) - (__popc(tracing) >> 2) >= (drained ? 1 : refill)) break;
-            if (phase == kTracing && !done && !quad_step<K, false>(P.accel, ro, rd, t, stack, P.error_word, ctr, ln, tracing)) {
+            if (phase == kTracing && !done && !quad_step<K, kSlack>(P.accel, ro, rd, t, stack, P.error_word, ctr, ln, tracing)) {
                 if (seeded && t.tk >= kFarT) {
                     seeded = false;
                     quad_continue(t, ctr);
@@ -1162,8 +1163,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_wb_replay(TraceParams P, BwdInp
 // that a round sets aside come in the order of the one-lane replay, so the same hits are scattered with the same
 // weights. Bound, as there, by the latency of a step, of which a job is a chain. Replay stage, against one lane a job:
 // 3.1 -> 2.4 ms (80k paths, 20k Gaussians), 4.9 -> 3.3 (90k, 100k), 7.3 -> 5.9 (90k, 300k); with 786k paths over
-// 1M Gaussians it took 41 ms against 18.6 (twice the frontier traffic an issue slot), hence the line.
-template <int K>
+// 1M Gaussians it took 41 ms against 18.6 (twice the frontier traffic an issue slot), hence the line. kSlack: with
+// the exact-candidate cull slack.
+template <int K, bool kSlack>
 __global__ void __maxnreg__(128) k_wb_replay_quad(TraceParams P, BwdInputs B, WfView W, unsigned cursor, int refill,
                                                  unsigned quad_jobs) {
     extern __shared__ float4 quad_mem[];
@@ -1220,7 +1222,8 @@ __global__ void __maxnreg__(128) k_wb_replay_quad(TraceParams P, BwdInputs B, Wf
         while (true) {
             const unsigned tracing = __ballot_sync(kFull, phase == kTracing);
             if (!tracing || __popc(busy) - (__popc(tracing) >> 2) >= (drained ? 1 : refill)) break;
-            if (phase == kTracing && !quad_step_resume<K>(P.accel, r.o, r.d, t, F, stack, P.error_word, ctr, ln, tracing))
+            if (phase == kTracing &&
+                !quad_step_resume<K, kSlack>(P.accel, r.o, r.d, t, F, stack, P.error_word, ctr, ln, tracing))
                 phase = kReady;
         }
         __syncwarp();  // the entries set aside, before the next call reads them
@@ -1236,14 +1239,22 @@ __global__ void __maxnreg__(128) k_wb_replay_quad(TraceParams P, BwdInputs B, Wf
     flush_counters(P, ctr);
 }
 
+// the four-lane replay, with the exact-candidate cull slack or without
+template <int K>
+static auto* replay_quad_fn(const WavefrontTuning& tune) {
+    return tune.exact_candidates ? k_wb_replay_quad<K, true> : k_wb_replay_quad<K, false>;
+}
+
 // persistent grid: resident blocks per SM x SMs (defined below)
 int grid_cached(const void* fn, int block, size_t smem);
 
 // The shadow stage with its own k-buffer size. A shadow walk visits the hits in distance order
 // until one occludes, whatever the batch size, so its size is free of the intersection's: a
 // walk usually ends in its first batch, which a smaller buffer gathers with less traversal.
-static void launch_shadow(int ks, const TraceParams& q, const WfView& W, int B, int R, const unsigned* items,
+static void launch_shadow(const WavefrontTuning& tune, const TraceParams& q, const WfView& W, const unsigned* items,
                           cudaStream_t s) {
+    const int B = tune.block, R = tune.refill_lanes;
+    const bool slack = tune.exact_candidates;
     // up to kQuadRays shadow rays (the queue's count, which only the device knows) go to the quads
     const auto blocks = [&](int grid, unsigned per_block) {
         return (unsigned)std::min<long long>(grid, ((long long)W.slots + per_block - 1) / per_block);
@@ -1255,10 +1266,10 @@ static void launch_shadow(int ks, const TraceParams& q, const WfView& W, int B, 
     const auto quads = [&](auto* fn) {
         fn<<<blocks(grid_cached((const void*)fn, B, stacks), B / 32), B, stacks, s>>>(q, W, (R + 3) / 4, W.q[kQShadow], kQuadRays);
     };
-    switch (ks) {
-    case 8: quads(k_wf_shadow_quad<8>); lanes(k_wf_shadow<8>, kQuadRays); break;
+    switch (tune.shadow_kbuf) {
+    case 8: quads(slack ? k_wf_shadow_quad<8, true> : k_wf_shadow_quad<8, false>); lanes(k_wf_shadow<8>, kQuadRays); break;
     case 32: lanes(k_wf_shadow<32>, 0u); break;
-    default: quads(k_wf_shadow_quad<16>); lanes(k_wf_shadow<16>, kQuadRays); break;
+    default: quads(slack ? k_wf_shadow_quad<16, true> : k_wf_shadow_quad<16, false>); lanes(k_wf_shadow<16>, kQuadRays); break;
     }
 }
 
@@ -1486,7 +1497,7 @@ static cudaError_t run_fwd(const TraceParams& p, const FwdOutputs& o, WavefrontB
     const unsigned chunk_tiles = (unsigned)std::min<unsigned long long>(tune.chunk_tiles, tiles);
     cudaError_t e = wavefront_reserve(b, (size_t)chunk_tiles * 32, s);
     if (e != cudaSuccess) return e;
-    const int B = tune.block, R = tune.refill_lanes;
+    const int B = tune.block;
     const int g_camera = grid_cached((const void*)k_wf_camera, B);
     const int g_primary = grid_cached((const void*)k_wf_fwd_primary<K>, B);
     const int g_bounce = grid_cached((const void*)k_wf_fwd_bounce<K>, B);
@@ -1513,7 +1524,7 @@ static cudaError_t run_fwd(const TraceParams& p, const FwdOutputs& o, WavefrontB
         if (p.flags & kMis) {
             const unsigned* shadow_items = sort_queue(p, b, W, tune, sc, s, tune.shadow_kbuf <= 16, kQShadow);
             sc.run(kStageShadow, p, s,
-                   [&](const TraceParams& q) { launch_shadow(tune.shadow_kbuf, q, W, B, R, shadow_items, s); });
+                   [&](const TraceParams& q) { launch_shadow(tune, q, W, shadow_items, s); });
         }
         unsigned cursor = kFirstBounceCursor;
         for (unsigned depth = 0; depth < mb; ++depth) {
@@ -1558,7 +1569,7 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
     const int g_replay = grid_cached((const void*)k_wb_replay<K>, B);
     int g_replay_quad = 0;
     if constexpr (K <= 16) {
-        if (resume_replay) g_replay_quad = grid_cached((const void*)k_wb_replay_quad<K>, B, quad_stacks);
+        if (resume_replay) g_replay_quad = grid_cached((const void*)replay_quad_fn<K>(tune), B, quad_stacks);
     }
     // frontiers: one a thread of a resumed kernel, one a quad of the replay
     const size_t fronts = std::max({resume ? (size_t)std::max(trace0.lane_grid, trace.lane_grid) * B : (size_t)0,
@@ -1585,7 +1596,7 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
         if (p.flags & kMis) {
             const unsigned* shadow_items = sort_queue(p, b, W, tune, sc, s, tune.shadow_kbuf <= 16, kQShadow);
             sc.run(kStageShadow, p, s,
-                   [&](const TraceParams& q) { launch_shadow(tune.shadow_kbuf, q, W, B, R, shadow_items, s); });
+                   [&](const TraceParams& q) { launch_shadow(tune, q, W, shadow_items, s); });
         }
         unsigned cursor = kFirstBounceCursor;
         for (unsigned depth = 0; depth < mb; ++depth) {
@@ -1599,7 +1610,7 @@ static cudaError_t run_bwd(const TraceParams& p, const BwdInputs& bi, WavefrontB
                 if constexpr (K <= 16) {
                     if (resume_replay) {
                         const long long need = (2ll * W.slots + B / 32 - 1) / (B / 32);
-                        k_wb_replay_quad<K><<<(unsigned)std::min<long long>(g_replay_quad, need), B, quad_stacks, s>>>(
+                        replay_quad_fn<K>(tune)<<<(unsigned)std::min<long long>(g_replay_quad, need), B, quad_stacks, s>>>(
                             q, bi, W, cursor, (R + 7) / 8, quad_jobs);
                     }
                 }
