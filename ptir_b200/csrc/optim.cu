@@ -21,8 +21,8 @@ __device__ __forceinline__ void adam_element(float g, float& p, float& m, float&
 }
 
 // One thread per four consecutive elements, read and written as 16 bytes each, whatever the row length: the four
-// may belong to two or more rows, and a hidden row's elements go back as they came. Nothing is read of a hidden
-// four but its rows' flags. Bound by HBM (28 bytes an element of a visible row); with one element a thread
+// may belong to two or more rows; of a four that spans a hidden row's border only the visible row's elements are
+// written. Nothing is read of a hidden four but its rows' flags. Bound by HBM (28 bytes an element of a visible row); with one element a thread
 // a 64-bit division by the row length each stood before the loads: 300,000 rows of 48, 60 % of them visible, took
 // 80.2 us and take 56.7 (242 MB, 4.3 TB/s). Index: unsigned while the elements fit.
 template <class Index>
@@ -54,9 +54,22 @@ __global__ void __launch_bounds__(256) k_selective_adam4(float4* __restrict__ pa
     if (on[1]) adam_element(g4.y, p4.y, m4.y, v4.y, lr, b1, b2, eps);
     if (on[2]) adam_element(g4.z, p4.z, m4.z, v4.z, lr, b1, b2, eps);
     if (on[3]) adam_element(g4.w, p4.w, m4.w, v4.w, lr, b1, b2, eps);
-    param[i] = p4;
-    m[i] = m4;
-    v[i] = v4;
+    if (on[0] && on[1] && on[2] && on[3]) {
+        param[i] = p4;
+        m[i] = m4;
+        v[i] = v4;
+        return;
+    }
+    // a row's border: the hidden elements may be another step's (of other rows, on another stream) and are not written
+    float *pe = reinterpret_cast<float*>(param + i), *me = reinterpret_cast<float*>(m + i), *ve = reinterpret_cast<float*>(v + i);
+    const float pa[4] = {p4.x, p4.y, p4.z, p4.w}, ma[4] = {m4.x, m4.y, m4.z, m4.w}, va[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (!on[k]) continue;
+        pe[k] = pa[k];
+        me[k] = ma[k];
+        ve[k] = va[k];
+    }
 }
 
 // one element per thread: the elements after the last four, and buffers that are not 16-byte aligned
