@@ -311,22 +311,28 @@ int ptirkat_kbuffer(int k, int form, int cases, int m, const float* ts, const un
 }
 
 // the tracer's radix sort of device buffers (keys of 32 or 64 bits, 32-bit values) by bits
-// [begin_bit, end_bit); 0 on success
-int ptirkat_radix_sort(int key_bytes, const void* keys_in, void* keys_out, const unsigned* vals_in, unsigned* vals_out,
-                       long long n, int begin_bit, int end_bit) {
+// [begin_bit, end_bit); with `count` (device) of the first *count items, and of none when they are `above` or fewer.
+// 0 on success
+int ptirkat_radix_sort_counted(int key_bytes, const void* keys_in, void* keys_out, const unsigned* vals_in,
+                               unsigned* vals_out, long long n, int begin_bit, int end_bit, const unsigned* count,
+                               unsigned above) {
     const size_t bytes = key_bytes == 8 ? radix_sort_temp_bytes<unsigned long long>(n) : radix_sort_temp_bytes<unsigned>(n);
     void* temp = nullptr;
     if (bytes && cudaMalloc(&temp, bytes) != cudaSuccess) return 1;
     cudaError_t e = key_bytes == 8
                         ? radix_sort_pairs<unsigned long long>(temp, bytes, static_cast<const unsigned long long*>(keys_in),
                                                                static_cast<unsigned long long*>(keys_out), vals_in, vals_out, n,
-                                                               begin_bit, end_bit, 0)
+                                                               begin_bit, end_bit, 0, count, above)
                         : radix_sort_pairs<unsigned>(temp, bytes, static_cast<const unsigned*>(keys_in),
                                                      static_cast<unsigned*>(keys_out), vals_in, vals_out, n, begin_bit,
-                                                     end_bit, 0);
+                                                     end_bit, 0, count, above);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (temp) cudaFree(temp);
     return e == cudaSuccess ? 0 : 1;
+}
+int ptirkat_radix_sort(int key_bytes, const void* keys_in, void* keys_out, const unsigned* vals_in, unsigned* vals_out,
+                       long long n, int begin_bit, int end_bit) {
+    return ptirkat_radix_sort_counted(key_bytes, keys_in, keys_out, vals_in, vals_out, n, begin_bit, end_bit, nullptr, 0u);
 }
 
 }  // extern "C"
