@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kPlocTailThreads) k_ploc_tail(int n, const uns
             if (i < count && sub == 0) T.nn[i] = best.other;
         }
         __syncthreads();
-        // merge mutual neighbours into the left one's place and compact, four consecutive clusters a thread
+        // merge mutual neighbours into the left one's place and compact, up to three consecutive clusters a thread
         const int per = (count + kPlocTailThreads - 1) / kPlocTailThreads;
         const int first = min(count, tid * per), last = min(count, first + per);
         unsigned kept = 0;

@@ -7,7 +7,7 @@
 // instructions an entry), every inserted (distance, id) is appended to a log in local memory, and the ids
 // are put in order once, when the call ends (near_resolve). With 16 registers less the kernel fits 72, seven blocks
 // of 128 threads an SM instead of five. Intersection stage of 786k paths over 1M Gaussians, forward and
-// adjoint: 147.5 -> 133.0 ms; of 627k over 600k: 72.4 -> 66.3. (With the children sorted by integer keys that hold the
+// adjoint: 147.5 -> 133.0 ms; of 627k over 600k: 72.3 -> 65.6. (With the children sorted by integer keys that hold the
 // child in their two lowest bits, in place of descend's whole keys: 135.1 and 67.8, and another order of close keys.)
 #pragma once
 
@@ -17,7 +17,7 @@ namespace ptir {
 
 // Log entries a lane, (distance bits, id) in insertion order. A full log drops what is past the K-th
 // distance: that leaves at most K - 1 nearer entries and K equal ones.
-// A call of 16 inserts about 34 entries. 34 entries of log: 136.5 ms in the stage at 1M Gaussians; 48: 135.0; 64: 134.7.
+// A call of 16 inserts about 34 entries. 34 entries of log: 133.9 ms in the stage at 1M Gaussians; 48: 133.0; 64: 132.4.
 constexpr int kNearLog = 48;
 
 template <int K>

@@ -7,7 +7,9 @@
 // the quad, and up to four stack entries are popped at a time. A visit decides what the one-lane visit
 // decides: the leaf tests of a node see the K-th distance as it was before the node, but an entry at or
 // past the current K-th distance enters the sorted buffer nowhere, which is the one-lane test's
-// rejection; children are visited and stacked in the same order.
+// rejection; children are visited and stacked in the same order (quad_order). What a small launch can differ in from a
+// large one is a grazing candidate: the one-lane kernels seed a first round's cut (wavefront.cu), the four-lane
+// ones do not.
 //
 // Bound: latency. A visit is a chain of a node load, box tests, leaf loads and tests, insertions and
 // the descent. With one lane a ray that chain took 0.9 to 1.2 us a visit (leaf tests one after the

@@ -1,5 +1,5 @@
 // Stable LSD radix sort of (key, value) pairs on the device: the sort of the LBVH build (60-bit
-// Morton keys) and of the wavefront's ray order (28-bit keys).
+// Morton keys) and of the wavefront's ray order (27-bit keys).
 //
 // Each pass sorts by one 8-bit digit. The items are split into warp tiles of consecutive items, 2048 or 512 of
 // them (rs_items). The number of items may be known on the device only (`count`, at most the host's n): tiles past

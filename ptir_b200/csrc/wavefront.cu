@@ -204,19 +204,7 @@ struct Parked {
     }
 };
 
-// Intersection stage: each lane carries one segment of queue `in_q` (read from `items`, the
-// queue in queue or sorted order) through as many trace calls as it needs (composite_begin /
-// trace / composite_hits / composite_end). A lane whose call has finished composites its batch
-// and starts the next call, or writes its segment, hands it to queue `out_q` (when >= 0) and
-// takes the next one from the queue, so that no lane waits for the slowest segment of its warp.
-// The warp leaves its traversal loop once `refill` lanes wait (a finished call, or idle while
-// the queue still holds segments). W.parked holds, per thread of the grid, the parked
-// accumulators and, while a batch is composited, its k-buffer (kParkedFields + 2K floats).
-//
-// Three kernels do this: k_wf_trace (two rounds a traversal with K = 32, and resumed rounds), k_wf_trace_near
-// (rounds from the root, K <= 16) and k_wf_trace_quad (the same, four lanes a ray, for small launches).
-//
-// Registers per thread of k_wf_trace (and of the shadow kernel of the same k-buffer size). The
+// Registers per thread of k_wf_trace (and of k_wf_shadow of the same k-buffer size). The
 // kernels use no shared memory, so registers alone set the resident warps. K <= 16: 96, five
 // 128-thread blocks per SM, 5 % faster than the compiler's own 127 (four blocks) despite a few
 // spills; 80 (six blocks) was 11 % slower (both measured on rounds from the root).
@@ -231,13 +219,25 @@ constexpr int trace_regs(int K) { return K > 16 ? 128 : 96; }
 // of them continued), against 145.5 ms at 1.5 and 143.2 ms at 3.
 constexpr float kSeedSpan = 2.0f;
 
-// Rays up to which an intersection launch takes four lanes a ray. Measured against one lane (the stage, ms):
-// 1.93 -> 0.93 at 16k rays over 10k Gaussians, 36.2 -> 23.3 at 90k over 300k. Where the line lies, against
-// k_wf_trace_near (lines at 65,536 / 94,720 / 131,072 / 262,144 rays): 8.0 / 7.9 / 7.5 / 7.5 at 278k primary
-// and 80k bounce rays over 30k Gaussians; 67.8 / 67.7 / 68.8 / 73.5 at 627k paths of several views over 600k;
-// 135.0 / 135.6 / 135.0 / 142.0 at 786k primary and about 200k bounce rays over 1M.
+// Rays up to which an intersection launch takes four lanes a ray. Measured against one lane with ids in registers (the
+// stage, ms): 1.92 -> 1.01 at 16k rays over 10k Gaussians, 37.2 -> 25.2 at 90k over 300k. Where the line lies,
+// against k_wf_trace_near (lines at 65,536 / 94,720 / 131,072 / 262,144 rays): 24.0 / 25.2 / 25.2 / 25.0 at 90k over
+// 300k and 12.5 / 11.5 / 11.5 / 11.6 at 90k over 100k; 7.8 / 7.7 / 7.5 / 7.6 at 278k primary and 80k bounce rays over
+// 30k; 65.7 / 66.2 / 65.6 / 73.1 at 627k paths of several views over 600k; 133.0 / 132.9 / 133.0 / 141.9 at 786k
+// primary and about 200k bounce rays over 1M.
 constexpr unsigned kQuadRays = 1u << 17;
 
+// Intersection stage: each lane carries one segment of queue `in_q` (read from `items`, the
+// queue in queue or sorted order) through as many trace calls as it needs (composite_begin /
+// trace / composite_hits / composite_end). A lane whose call has finished composites its batch
+// and starts the next call, or writes its segment, hands it to queue `out_q` (when >= 0) and
+// takes the next one from the queue, so that no lane waits for the slowest segment of its warp.
+// The warp leaves its traversal loop once `refill` lanes wait (a finished call, or idle while
+// the queue still holds segments). W.parked holds, per thread of the grid, the parked
+// accumulators and, while a batch is composited, its k-buffer (kParkedFields + 2K floats).
+//
+// Three kernels do this: k_wf_trace (two rounds a traversal with K = 32, and resumed rounds), k_wf_trace_near
+// (rounds from the root, K <= 16) and k_wf_trace_quad (the same, four lanes a ray, for small launches).
 //
 // With K = 32 a traversal stands for two of the reference's 16-candidate rounds (the rounds of
 // pathTracer.cuh:216-311): its first 16 candidates are the first round, and its last 16 are the
@@ -399,8 +399,8 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_trace(TraceParams P, float* vis,
 }
 
 // k_wf_trace for the rounds from the root (K <= 16), with the k-buffer of near.cuh: the same calls, seeds and
-// compositing. 72 registers: on 786k paths over 1M Gaussians (forward and adjoint) the stage took 135.3 ms, against
-// 139.2 at 80, 151.1 at 64 and 178.0 at 56.
+// compositing. 72 registers: on 786k paths over 1M Gaussians (forward and adjoint) the stage took 133.0 ms, against
+// 137.5 at 80, 144.6 at 64 and 168.5 at 56.
 template <int K, bool kMark, bool kSelfOcc, bool kSlack>
 __global__ void __maxnreg__(72) k_wf_trace_near(TraceParams P, float* vis, WfView W, int in_q, const unsigned* items,
                                                 int out_q, unsigned cursor, int refill, unsigned quad_rays) {
@@ -548,8 +548,8 @@ PTIR_DEV unsigned quads_in_use(unsigned count) {
 // The decisions, their order and the compositing are k_wf_trace_near's, and no first round is seeded: a quad rarely
 // sees more than a few segments. A small launch is bound by the chain of its slowest ray, which one lane walks
 // at about 1 us a visit; here the visit's parts run side by side (preview of 2,867 rays over 2k Gaussians:
-// 1.42 -> 0.49 ms in the stage). 96 registers hold the visit without spills: 23.6 ms at 90k rays over 300k
-// Gaussians, against 26.1 at 72 and 25.9 at 64, where spills cost more than the warps gain.
+// 1.41 -> 0.51 ms in the stage). 96 registers hold the visit without spills: 25.2 ms at 90k rays over 300k
+// Gaussians, against 26.1 at 72 and 26.9 at 64, where spills cost more than the warps gain, and 27.8 at 128.
 template <int K, bool kMark, bool kSelfOcc, bool kSlack>
 __global__ void __maxnreg__(96) k_wf_trace_quad(TraceParams P, float* vis, WfView W, int in_q, const unsigned* items,
                                                 int out_q, unsigned cursor, int refill, unsigned quad_rays) {
@@ -895,7 +895,7 @@ __global__ void __maxnreg__(trace_regs(K)) k_wf_shadow(TraceParams P, WfView W, 
 
 // k_wf_shadow for small launches, a quad of lanes a ray (quad.cuh): the same candidates, walked in the same order with
 // the same draws; no first round is seeded, as in k_wf_trace_quad. As there a small launch waits for its slowest
-// ray: stage of 16k rays over 10k Gaussians 0.60 -> 0.26 ms, of 90k over 300k (forward and adjoint) 6.6 -> 4.1 ms.
+// ray: stage of 16k rays over 10k Gaussians 0.57 -> 0.26 ms, of 90k over 300k (forward and adjoint) 6.4 -> 4.2 ms.
 // kSlack: with the exact-candidate cull slack.
 template <int K, bool kSlack>
 __global__ void __maxnreg__(96) k_wf_shadow_quad(TraceParams P, WfView W, int refill, const unsigned* items,
@@ -1162,7 +1162,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_wb_replay(TraceParams P, BwdInp
 // k_wb_replay with resumed rounds (K <= 16) for up to kQuadRays jobs, a quad of lanes a job (quad.cuh): the entries
 // that a round sets aside come in the order of the one-lane replay, so the same hits are scattered with the same
 // weights. Bound, as there, by the latency of a step, of which a job is a chain. Replay stage, against one lane a job:
-// 3.1 -> 2.4 ms (80k paths, 20k Gaussians), 4.9 -> 3.3 (90k, 100k), 7.3 -> 5.9 (90k, 300k); with 786k paths over
+// 3.2 -> 2.6 ms (80k paths, 20k Gaussians), 4.9 -> 3.4 (90k, 100k), 7.0 -> 6.1 (90k, 300k); with 786k paths over
 // 1M Gaussians it took 41 ms against 18.6 (twice the frontier traffic an issue slot), hence the line. kSlack: with
 // the exact-candidate cull slack.
 template <int K, bool kSlack>

@@ -97,8 +97,9 @@ class OptixTracer:
     traversal; 16 and 32 composite in the reference's rounds of 16, a 32-entry traversal standing
     for two rounds when its second half is the next round's candidates), ``refill_lanes`` (waiting lanes before an intersection warp refills, 1..32) and
     ``block_size`` (64, 128 or 256); 0 keeps the default. ``collect_timings`` records CUDA events
-    around every kernel launch for ``stage_times()``; ``sort_rays`` intersects bounce rays in
-    (direction octant, origin cell, direction cell) order (the results do not change); ``exact_replay`` lets the
+    around every kernel launch for ``stage_times()``; ``sort_rays`` intersects bounce and shadow rays in
+    (direction octant, origin cell, direction cell) order, in launches of more than 131,072 rays (the results do not
+    change, up to the grazing candidates that depend on the traversal's order: ``exact_candidates``); ``exact_replay`` lets the
     backward re-traversals include each segment's last composited Gaussian, which the
     reference's float epsilon leaves out; ``compensated_grads``
     accumulates the gradient atomics as Kahan pairs (off: plain float atomics, as the
