@@ -2,7 +2,8 @@
 // evaluates hit 4r + c of round r (the particle response and what the hit contributes, none of which
 // depends on the hits before it), then the quad goes over the four hits in order. The order-dependent
 // part (transmittance, acceptance while it lasts, the sums) is composite_one's, operation for operation,
-// so the sums are bitwise those of one lane going over the batch.
+// so the sums are those of one lane going over the batch, up to how the compiler contracts a term's multiply-adds (with a
+// k-buffer of 8 and SH of degree 3 the radiance differs in its last bit, and is the megakernel's).
 #pragma once
 
 #include "path.cuh"
